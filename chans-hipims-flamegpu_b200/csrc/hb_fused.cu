@@ -537,31 +537,57 @@ finish_kernel(const hb_instance *__restrict__ insts, BcTable *__restrict__ bct,
   advance_clock<T, kNT>(in, blockIdx.x, bct, sm, dry != 0.0 ? 1 : 0, in.ctrl);
 }
 
-// Workspace layout (each part 256-byte aligned): [n_tiles] TilePartial,
-// [n_groups] TilePartial (sums of groups of kGroupTiles tiles), [n_groups]
-// unsigned group counters, [n_tiles] int32 tile order (rows kernel: general
-// tiles, then all-valid tiles), [2] int32 counts of the two, [n_tiles] uint8
-// all-valid flags, 64-wide tiles only: [n_tiles] TileEntry in the order's
-// order, then [n_instances] BcTable, then [n_instances][kMapsPerInstance]
-// CUtensorMap.  Instance i's groups start at tile_begin / kGroupTiles + i,
-// which never overlaps instance i + 1's.
+// Rows of the blocks a step's CTAs take.  A tile is the unit of the caller's
+// grid (tiles_x, tiles_y, tile_begin); where a batch has so few tiles that
+// whole tiles leave the chip's CTA slots idle, every tile is divided into
+// tile_y / step_rows(b) blocks of that many rows, each its own CTA with its
+// own class, list entry and partial sums.  Depends on the batch record alone,
+// so that the workspace size, prepare and every step agree.
+// 64-wide FP32 tiles: a CTA's time is its warps' serial walk (8 rows a warp in
+// a 32-row tile, about 1 us a row when the SM holds one CTA), so below one wave
+// of whole tiles 8-row blocks (2 rows a warp) finish sooner although every
+// band start costs an extra row of y-faces.
+constexpr int kDividePairsTiles = 592;
+inline int step_rows(const hb_fused_batch *b) {
+  if (b->flags & (HB_FLAG_TILE_TASKS | HB_FLAG_WHOLE_TILES)) return b->tile_y;
+  if (b->tile_x == 64 && b->tile_y == 32 && b->n_tiles <= kDividePairsTiles) return 8;
+  return b->tile_y;
+}
+inline int blocks_per_tile(const hb_fused_batch *b) {
+  const int r = step_rows(b);
+  return r > 0 ? b->tile_y / r : 1;
+}
+inline int n_blocks(const hb_fused_batch *b) {
+  return b->n_tiles * std::max(blocks_per_tile(b), 1);
+}
+
+// Workspace layout (each part 256-byte aligned), n = n_blocks: [n]
+// TilePartial, [n_groups] TilePartial (sums of groups of kGroupTiles blocks),
+// [n_groups] unsigned group counters, [n] int32 block order (rows kernel:
+// general blocks, then all-valid blocks), [3] int32 counts, [n] uint8
+// all-valid flags, 64-wide tiles only: [n] TileEntry in the order's order,
+// then [n_instances] BcTable, then [n_instances][kMapsPerInstance]
+// CUtensorMap.  Instance i's groups start at (its first block) / kGroupTiles
+// + i, which never overlaps instance i + 1's.
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-inline size_t ws_partials_bytes(int n_tiles) { return align256((size_t)n_tiles * sizeof(TilePartial)); }
+inline size_t ws_partials_bytes(const hb_fused_batch *b) {
+  return align256((size_t)n_blocks(b) * sizeof(TilePartial));
+}
 inline int ws_n_groups(const hb_fused_batch *b) {
-  return b->n_tiles / kGroupTiles + b->n_instances + 1;
+  return n_blocks(b) / kGroupTiles + b->n_instances + 1;
 }
 inline size_t ws_gcount_offset(const hb_fused_batch *b) {
-  return ws_partials_bytes(b->n_tiles) + align256((size_t)ws_n_groups(b) * sizeof(TilePartial));
+  return ws_partials_bytes(b) + align256((size_t)ws_n_groups(b) * sizeof(TilePartial));
 }
 inline size_t ws_order_offset(const hb_fused_batch *b) {
   return ws_gcount_offset(b) + align256((size_t)ws_n_groups(b) * sizeof(unsigned));
 }
 inline size_t ws_counts_offset(const hb_fused_batch *b) {
-  return ws_order_offset(b) + align256((size_t)b->n_tiles * sizeof(int32_t));
+  return ws_order_offset(b) + align256((size_t)n_blocks(b) * sizeof(int32_t));
 }
 inline size_t ws_flags_offset(const hb_fused_batch *b) { return ws_counts_offset(b) + 256; }
-// What a tile of the two-cells-per-lane step needs before it can issue its
-// tile loads, in one 16-byte record: the tile (~tile when it holds no valid
+// What a block of the two-cells-per-lane step needs before it can issue its
+// loads, in one 16-byte record: the block (~block when it holds no valid
 // cell), its instance and that instance's control block.
 struct alignas(16) TileEntry {
   int32_t tile;
@@ -570,10 +596,10 @@ struct alignas(16) TileEntry {
 };
 static_assert(sizeof(TileEntry) == 16, "one 16-byte load per tile");
 inline size_t ws_entries_offset(const hb_fused_batch *b) {
-  return ws_flags_offset(b) + align256((size_t)b->n_tiles);
+  return ws_flags_offset(b) + align256((size_t)n_blocks(b));
 }
 inline size_t ws_entries_bytes(const hb_fused_batch *b) {
-  return b->tile_x == 64 ? align256((size_t)b->n_tiles * sizeof(TileEntry)) : 0;
+  return b->tile_x == 64 ? align256((size_t)n_blocks(b) * sizeof(TileEntry)) : 0;
 }
 inline size_t ws_bct_offset(const hb_fused_batch *b) {
   return ws_entries_offset(b) + ws_entries_bytes(b);
@@ -1768,14 +1794,14 @@ int launch_steps(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
 // cell is out of its reach; the rows kernel runs those tiles in its all-valid
 // build and the others in its general build.
 // ---------------------------------------------------------------------------
-template <int TY, int TW>
+template <int TY, int TW, int PER = 1>
 __global__ void __launch_bounds__(kRowsNT)
 classify_tiles_kernel(const hb_instance *__restrict__ insts, const int32_t *__restrict__ tile_inst,
                       int n_tiles, uint8_t *__restrict__ flags) {
-  const int tile = blockIdx.x;
+  const int tile = blockIdx.x;  // a tile, or one of its PER blocks of TY rows
   if (tile >= n_tiles) return;
-  const hb_instance &in = insts[tile_inst[tile]];
-  const int lt = tile - in.tile_begin;
+  const hb_instance &in = insts[tile_inst[tile / PER]];
+  const int lt = tile - in.tile_begin * PER;
   const int tyi = lt / in.tiles_x, txi = lt - tyi * in.tiles_x;
   const int y0 = tyi * TY, x0 = txi * TW;
   bool ok = !(in.bug_y >= y0 - 2 && in.bug_y <= y0 + TY + 1 && in.bug_x >= x0 - 4 &&
@@ -1860,13 +1886,13 @@ order_tiles_kernel(const uint8_t *__restrict__ flags, int n, int32_t *__restrict
 
 // The order as TileEntry records (64-wide tiles): entries[k] for order[k].
 __global__ void __launch_bounds__(256)
-tile_entries_kernel(const int32_t *__restrict__ order, int n,
+tile_entries_kernel(const int32_t *__restrict__ order, int n, int per,
                     const int32_t *__restrict__ tile_inst, const hb_instance *__restrict__ insts,
                     TileEntry *__restrict__ entries) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int e = order[k];
-  const int ii = tile_inst[e < 0 ? ~e : e];
+  const int ii = tile_inst[(e < 0 ? ~e : e) / per];
   TileEntry r;
   r.tile = e;
   r.inst = ii;
@@ -1945,7 +1971,7 @@ int launch_rows_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   const int grid_g = b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : std::min(n_general, n);
   char *ws = reinterpret_cast<char *>(b->workspace);
   TilePartial *parts = reinterpret_cast<TilePartial *>(ws);
-  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b->n_tiles));
+  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b));
   unsigned *gcount = reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b));
   const int32_t *order = reinterpret_cast<const int32_t *>(ws + ws_order_offset(b));
   const int32_t *counts = reinterpret_cast<const int32_t *>(ws + ws_counts_offset(b));
@@ -1974,14 +2000,46 @@ int launch_rows_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
 // both at once; the general build keeps the register cap of 3 CTAs per SM
 // (its ghost-face branches spill under a tighter one) and MINB caps the
 // all-valid build.
-template <int TY, int MINB, bool SOURCES, int ORDER = 2>
-int launch_pairs_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
+template <int TY, bool SOURCES, int ORDER>
+int launch_mixed(const hb_fused_batch *b, int nsteps, int grid, int n_live, int n_valid_end, int n,
+                 cudaStream_t st) {
   using S = PairSmem<TY>;
-  const int n = b->n_tiles;
+  auto *km = pairs_mixed_kernel<TY, SOURCES, ORDER>;
+  const int rc = set_smem_attr(reinterpret_cast<const void *>(km), (int)sizeof(S));
+  if (rc) return rc;
+  char *ws = reinterpret_cast<char *>(b->workspace);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::max(grid, 1));
+  cfg.blockDim = dim3(kRowsNT);
+  cfg.dynamicSmemBytes = sizeof(S);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  for (int k = 0; k < nsteps; k++) {
+    const cudaError_t e = cudaLaunchKernelEx(
+        &cfg, km, b->instances, reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b)),
+        n_live, n_valid_end, n, reinterpret_cast<TilePartial *>(ws),
+        reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b)),
+        reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b)),
+        reinterpret_cast<BcTable *>(ws + ws_bct_offset(b)),
+        reinterpret_cast<const CUtensorMap *>(ws + ws_maps_offset(b)));
+    if (e != cudaSuccess) return set_error(HB_ERR_CUDA, "hb_fused_step: %s", cudaGetErrorString(e));
+  }
+  return check_launch("hb_fused_step");
+}
+
+template <int MINB, bool SOURCES, int ORDER = 2>
+int launch_pairs_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
+  constexpr int TY = 32;
+  using S = PairSmem<TY>;
+  const int n = n_blocks(b);
   // the list lengths come from prepare (one read-back there), so that a
-  // tile's first load is its own entry
-  // entries: general tiles with a valid cell [0, n_live), all-valid tiles
-  // [n_live, n_live + n_valid), tiles without a valid cell [.., n)
+  // block's first load is its own entry
+  // entries: general blocks with a valid cell [0, n_live), all-valid blocks
+  // [n_live, n_live + n_valid), blocks without a valid cell [.., n)
   int n_general = 0, n_empty = 0;
   {
     std::lock_guard<std::mutex> lock(g_side_mu);
@@ -1992,23 +2050,20 @@ int launch_pairs_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
     n_empty = std::min(std::max(it->second.empty, 0), n_general);
   }
   const int n_valid = n - n_general, n_live = n_general - n_empty;
+  // 8-row blocks (a small batch): one launch whatever the register cap asked for
+  if (step_rows(b) == 8)
+    return launch_mixed<8, SOURCES, ORDER>(
+        b, nsteps, b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : n, n_live, n_live + n_valid,
+        n, st);
+  if (MINB == 4 && b->grid_blocks <= 0)
+    return launch_mixed<TY, SOURCES, ORDER>(b, nsteps, n, n_live, n_live + n_valid, n, st);
   char *ws = reinterpret_cast<char *>(b->workspace);
   TilePartial *parts = reinterpret_cast<TilePartial *>(ws);
-  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b->n_tiles));
+  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b));
   unsigned *gcount = reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b));
   const TileEntry *entries = reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b));
   BcTable *bct = reinterpret_cast<BcTable *>(ws + ws_bct_offset(b));
   const CUtensorMap *maps = reinterpret_cast<const CUtensorMap *>(ws + ws_maps_offset(b));
-  if (MINB == 4 && b->grid_blocks <= 0) {
-    auto *km = pairs_mixed_kernel<TY, SOURCES, ORDER>;
-    const int rc = set_smem_attr(reinterpret_cast<const void *>(km), (int)sizeof(S));
-    if (rc) return rc;
-    for (int k = 0; k < nsteps; k++)
-      km<<<std::max(n, 1), kRowsNT, sizeof(S), st>>>(b->instances, entries, n_live,
-                                                     n_live + n_valid, n, parts, gparts, gcount,
-                                                     bct, maps);
-    return check_launch("hb_fused_step");
-  }
   auto *kg = pairs_step_kernel<TY, 3, SOURCES, 0, ORDER>;
   auto *ka = pairs_step_kernel<TY, MINB, SOURCES, 1, ORDER>;
   int rc = set_smem_attr(reinterpret_cast<const void *>(kg), (int)sizeof(S));
@@ -2043,15 +2098,15 @@ int launch_pairs(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   const int minb = (b->flags >> HB_FLAG_MINB_SHIFT) & 0xF;
   const bool src = (b->flags & HB_FLAG_SOURCES) != 0;
   if (b->order == 1) {  // the 1st-order scheme: the all-valid build at 4 CTAs per SM
-    if (minb == 0 || minb == 4) return src ? launch_pairs_impl<32, 4, true, 1>(b, nsteps, st)
-                                           : launch_pairs_impl<32, 4, false, 1>(b, nsteps, st);
+    if (minb == 0 || minb == 4) return src ? launch_pairs_impl<4, true, 1>(b, nsteps, st)
+                                           : launch_pairs_impl<4, false, 1>(b, nsteps, st);
     return set_error(HB_ERR_ARG, "hb_fused_step: the 1st-order 64-wide tiles are built for "
                                  "4 CTAs per SM (minb 0 or 4), not %d", minb);
   }
-  if (minb == 3) return src ? launch_pairs_impl<32, 3, true>(b, nsteps, st)
-                            : launch_pairs_impl<32, 3, false>(b, nsteps, st);
-  if (minb == 0 || minb == 4) return src ? launch_pairs_impl<32, 4, true>(b, nsteps, st)
-                                         : launch_pairs_impl<32, 4, false>(b, nsteps, st);
+  if (minb == 3) return src ? launch_pairs_impl<3, true>(b, nsteps, st)
+                            : launch_pairs_impl<3, false>(b, nsteps, st);
+  if (minb == 0 || minb == 4) return src ? launch_pairs_impl<4, true>(b, nsteps, st)
+                                         : launch_pairs_impl<4, false>(b, nsteps, st);
   return set_error(HB_ERR_ARG, "hb_fused_step: 64-wide tiles are built for 3 or 4 CTAs per SM "
                                "(minb 0, 3 or 4), not %d", minb);
 }
@@ -2110,7 +2165,7 @@ int encode_2d(CUtensorMap *map, CUtensorMapDataType dt, size_t esize, const void
 // Host records are read from b->instances_host.
 int encode_maps(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_maps) {
   if (!b->instances_host) return set_error(HB_ERR_ARG, "hb_fused_prepare: instances_host is null");
-  const int TY = b->tile_y;
+  const int TY = step_rows(b);
   const int TW = b->tile_x;  // 32 (rows kernel) or 64 (two cells per lane)
   const size_t es = b->dtype == HB_F64 ? 8 : 4;
   const CUtensorMapDataType dt =
@@ -2120,7 +2175,7 @@ int encode_maps(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_maps
   for (int i = 0; i < b->n_instances; i++) {
     const hb_instance &in = b->instances_host[i];
     const uint64_t rows_s = (uint64_t)((in.rows + 63) / 64 * 64 + 2 * HB_PAD_Y);
-    if ((int64_t)in.tiles_y * TY + 4 > (int64_t)rows_s || in.tiles_x * TW + 8 > in.pitch ||
+    if ((int64_t)in.tiles_y * b->tile_y + 4 > (int64_t)rows_s || in.tiles_x * TW + 8 > in.pitch ||
         in.tiles_x * TW + 32 > in.code_pitch)
       return set_error(HB_ERR_ARG, "instance %d: storage smaller than its tiles", i);
     CUtensorMap *m = &maps[(size_t)i * kMapsPerInstance];
@@ -2215,7 +2270,11 @@ int prepare_impl(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_map
     if (rc) return rc;
     char *ws = reinterpret_cast<char *>(b->workspace);
     uint8_t *flags = reinterpret_cast<uint8_t *>(ws + ws_flags_offset(b));
-    if (b->tile_x == kPW)
+    const int n = n_blocks(b), per = blocks_per_tile(b);
+    if (b->tile_x == kPW && per == 4)
+      classify_tiles_kernel<8, kPW, 4><<<n, kRowsNT, 0, st>>>(b->instances, b->tile_instance, n,
+                                                              flags);
+    else if (b->tile_x == kPW)
       classify_tiles_kernel<32, kPW><<<b->n_tiles, kRowsNT, 0, st>>>(
           b->instances, b->tile_instance, b->n_tiles, flags);
     else if (b->tile_y == 64)
@@ -2225,12 +2284,12 @@ int prepare_impl(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_map
       classify_tiles_kernel<32, kTW><<<b->n_tiles, kRowsNT, 0, st>>>(
           b->instances, b->tile_instance, b->n_tiles, flags);
     order_tiles_kernel<<<1, kOrderNT, 0, st>>>(
-        flags, b->n_tiles, reinterpret_cast<int32_t *>(ws + ws_order_offset(b)),
+        flags, n, reinterpret_cast<int32_t *>(ws + ws_order_offset(b)),
         reinterpret_cast<int32_t *>(ws + ws_counts_offset(b)));
     if (b->tile_x == kPW)
-      tile_entries_kernel<<<(b->n_tiles + 255) / 256, 256, 0, st>>>(
-          reinterpret_cast<const int32_t *>(ws + ws_order_offset(b)), b->n_tiles,
-          b->tile_instance, b->instances, reinterpret_cast<TileEntry *>(ws + ws_entries_offset(b)));
+      tile_entries_kernel<<<(n + 255) / 256, 256, 0, st>>>(
+          reinterpret_cast<const int32_t *>(ws + ws_order_offset(b)), n, per, b->tile_instance,
+          b->instances, reinterpret_cast<TileEntry *>(ws + ws_entries_offset(b)));
     int32_t counts[3] = {0, 0, 0};
     cudaError_t e = cudaMemcpyAsync(counts, ws + ws_counts_offset(b), sizeof(counts),
                                     cudaMemcpyDeviceToHost, st);
@@ -2408,7 +2467,11 @@ extern "C" int hb_fused_step_noalloc(const hb_fused_batch *b, int nsteps, int pr
     return set_error(HB_ERR_ARG, "hb_fused_step_noalloc: bad batch record");
   hb_fused_batch local = *b;
   local.workspace = nullptr;
-  const size_t need = hb_fused_workspace_size(&local);
+  size_t need = hb_fused_workspace_size(&local);
+  if (need > kNoAllocScratchBytes) {  // whole tiles need the smaller workspace
+    local.flags |= HB_FLAG_WHOLE_TILES;
+    need = hb_fused_workspace_size(&local);
+  }
   if (need > kNoAllocScratchBytes)
     return set_error(HB_ERR_LIMIT,
                      "hb_fused_step_noalloc: this batch needs %zu bytes of scratch; the fixed "
@@ -2454,10 +2517,10 @@ extern "C" int hb_fused_step_noalloc(const hb_fused_batch *b, int nsteps, int pr
 namespace hb {
 namespace {
 
-template <bool SOURCES>
+template <int TY, bool SOURCES>
 int launch_persistent(const hb_fused_batch *b, int nsteps, long long budget, cudaStream_t st) {
-  using S = PairSmem<32>;
-  auto *kern = pairs_persistent_kernel<32, SOURCES>;
+  using S = PairSmem<TY>;
+  auto *kern = pairs_persistent_kernel<TY, SOURCES>;
   int rc = set_smem_attr(reinterpret_cast<const void *>(kern), (int)sizeof(S));
   if (rc) return rc;
   int per_sm = 0;
@@ -2466,14 +2529,14 @@ int launch_persistent(const hb_fused_batch *b, int nsteps, long long budget, cud
     return set_error(HB_ERR_CUDA, "hb_fused_run: occupancy: %s",
                      e != cudaSuccess ? cudaGetErrorString(e) : "no resident block");
   int grid = per_sm * num_sms();
-  if (grid > b->n_tiles) grid = b->n_tiles;
+  if (grid > n_blocks(b)) grid = n_blocks(b);
   char *ws = reinterpret_cast<char *>(b->workspace);
   const hb_instance *insts = b->instances;
   const TileEntry *entries = reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b));
   const int32_t *counts = reinterpret_cast<const int32_t *>(ws + ws_counts_offset(b));
   const uint8_t *allvalid = reinterpret_cast<const uint8_t *>(ws + ws_flags_offset(b));
   TilePartial *parts = reinterpret_cast<TilePartial *>(ws);
-  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b->n_tiles));
+  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b));
   unsigned *gcount = reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b));
   BcTable *bct = reinterpret_cast<BcTable *>(ws + ws_bct_offset(b));
   const CUtensorMap *maps = reinterpret_cast<const CUtensorMap *>(ws + ws_maps_offset(b));
@@ -2507,6 +2570,10 @@ extern "C" int hb_fused_run(const hb_fused_batch *b, int nsteps, long long budge
   if (nsteps == 0) return HB_OK;
   const long long budget = budget_cycles > 0 ? budget_cycles : (1LL << 31);
   auto st = as_stream(stream);
-  if (b->flags & HB_FLAG_SOURCES) return launch_persistent<true>(b, nsteps, budget, st);
-  return launch_persistent<false>(b, nsteps, budget, st);
+  const bool src = (b->flags & HB_FLAG_SOURCES) != 0;
+  if (step_rows(b) == 8)
+    return src ? launch_persistent<8, true>(b, nsteps, budget, st)
+               : launch_persistent<8, false>(b, nsteps, budget, st);
+  return src ? launch_persistent<32, true>(b, nsteps, budget, st)
+             : launch_persistent<32, false>(b, nsteps, budget, st);
 }

@@ -541,6 +541,7 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
                                           const CUtensorMap *__restrict__ maps) {
   constexpr bool kAllValid = PATH == 1;
   constexpr bool ALLV = kAllValid;
+  constexpr int kPer = 32 / TY;  // blocks of TY rows per 32-row tile
   const bool skip = !kAllValid && en.tile < 0;
   const int tile = en.tile < 0 ? ~en.tile : en.tile;
   using S = PairSmem<TY>;
@@ -551,7 +552,8 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
   const hb_instance &in = insts[ii];
   hb_ctrl *ctrl = en.ctrl;
   if (__ldcg(&ctrl->halted)) return true;
-  const int lt = tile - in.tile_begin;
+  const int tile0 = in.tile_begin * kPer;  // the instance's first block
+  const int lt = tile - tile0;
   const int tyi = lt / in.tiles_x, txi = lt - tyi * in.tiles_x;
   const int y0 = tyi * TY, x0 = txi * kPW;
   // the control block changes between steps (a persistent launch reads it
@@ -1006,10 +1008,10 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
     s.red_i[w] = any_dry;
   }
   __syncthreads();
-  const int n_inst_tiles = in.tiles_x * in.tiles_y;
+  const int n_inst_tiles = in.tiles_x * in.tiles_y * kPer;
   const int grp = lt / kGroupTiles;
   const int gsize = min(kGroupTiles, n_inst_tiles - grp * kGroupTiles);
-  const int gbase = in.tile_begin / kGroupTiles + ii;
+  const int gbase = tile0 / kGroupTiles + ii;
   if (tid == 0) {
     TilePartial p;
     p.volume = p.outflow = p.smax = 0.0;
@@ -1027,8 +1029,8 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
   }
   __syncthreads();
   if (s.last)
-    close_group<float, kRowsNT>(in, ii, partials + in.tile_begin + grp * kGroupTiles, gsize,
-                                gparts, gcount, gbase + grp, gbase,
+    close_group<float, kRowsNT>(in, ii, partials + tile0 + grp * kGroupTiles, gsize, gparts,
+                                gcount, gbase + grp, gbase,
                                 (n_inst_tiles + kGroupTiles - 1) / kGroupTiles, bct, s.red_d,
                                 s.red_s, s.red_i, &s.last2);
   __syncthreads();
@@ -1116,12 +1118,30 @@ pairs_mixed_kernel(const hb_instance *__restrict__ insts, const TileEntry *__res
   using S = PairSmem<TY>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   S &s = *reinterpret_cast<S *>(smem_raw);
+  // Programmatic launch: the next kernel's CTAs may take their slots once every
+  // CTA of this grid has started, and this one waits here for the kernel before
+  // it; everything that kernel may have written is read after the wait.  Hides
+  // the launch gap: 90.1 -> 87.7 us a step on 2048^2, 27.2 -> 25.7 on 256^2.
+  asm volatile("griddepcontrol.launch_dependents;");
   if (threadIdx.x == 0) {
     mbar_init(&s.bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   unsigned phase = 0;
+  if constexpr (TY != 32) {
+    for (int k = blockIdx.x; k < n_list; k += gridDim.x) {
+      const bool ok = k >= n_live && k < n_valid_end
+                          ? pair_tile<TY, SOURCES, 1, ORDER>(s, phase, list[k], insts, partials,
+                                                             gparts, gcount, bct, maps)
+                          : pair_tile_general<TY, SOURCES, ORDER>(s, phase, list[k], insts,
+                                                                  partials, gparts, gcount, bct,
+                                                                  maps);
+      if (!ok) return;
+    }
+    return;
+  }
   const int k = blockIdx.x;
   if (k < n_live || (k >= n_valid_end && k < n_list)) {
     pair_tile_general<TY, SOURCES, ORDER>(s, phase, list[k], insts, partials, gparts, gcount,

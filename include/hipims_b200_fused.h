@@ -43,6 +43,10 @@ extern "C" {
 /* hb_fused_batch.flags: some instance has infiltration or station rain (the
  * rows kernel build with those source terms; hb_fused_prepare checks it). */
 #define HB_FLAG_SOURCES 4
+/* hb_fused_batch.flags: one CTA per tile however few tiles there are (by
+ * default the tiles of a small batch are divided into shorter blocks, which
+ * takes a larger workspace).  Set it before hb_fused_workspace_size. */
+#define HB_FLAG_WHOLE_TILES 8
 /* hb_fused_batch.flags bits 8-11: register cap of the rows kernel expressed
  * as resident CTAs per SM (0 = compiler default; 5, 6 for 32-row tiles; 4 for
  * 64-row tiles).  The autotuner picks it. */
