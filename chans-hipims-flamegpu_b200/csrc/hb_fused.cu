@@ -50,7 +50,7 @@ constexpr int kNT = 256;  // threads per CTA
 // the last group of an instance finalizes the step from the group sums.
 constexpr int kGroupTiles = 128;
 
-struct TilePartial {
+struct alignas(16) TilePartial {  // read as two 16-byte words (add_partial)
   double smax;     // max CFL wave speed sqrt(g h) + max(|qx|, |qy|) / h over wet cells
   double volume;   // sum of h over valid cells
   double outflow;  // sum over boundary faces of the outward mass flux
@@ -303,31 +303,116 @@ __device__ void bc_values_exact(const hb_instance &in, double t, BcTable *out) {
 }
 
 
-// Last tile of an instance in a step: reduce the tiles' partials and advance
-// the control block (HP/SWE_CUDA.py:818-831): dt = min over cells of
-// CFL * dx / speed (60 s for dry cells), the 10x growth cap, the clip to the
-// next export time, t += dt, FP64 volume / outflow / rain totals, and the rain
-// rate and boundary values of the next step.  Called by every thread of the
-// CTA that finished the instance's last tile.
+// ---------------------------------------------------------------------------
+// The end of a step: the block that finishes an instance's last tile reduces
+// the partials, accounts the step's volumes, flips the state buffer and
+// advances the clock.  It runs after the last wave with the rest of the chip
+// idle, so it is bound by the length of its chain of dependent L2 round trips
+// (about 0.4 us each).  Everything that does not depend on the reduced wave
+// speed (control block, instance record, the rain rows around the cursor, the
+// boundary tables' times) is therefore loaded beside the partials, one role
+// per warp, and up to kOneGroupTiles tiles are summed in one level.  From the
+// last tile's count to the new clock 10.4-13 k cycles (5-6.5 us) before and
+// about 6 k after in one level; a step of 256^2 went from 18.4 to 16.0 us.
+// close_group is kept out of line: inlined, it cost the all-valid tiles of the
+// FP32 step 0.5-3 % through their register allocation.
+// ---------------------------------------------------------------------------
+
+// What each role of the clock holds before the wave speed is known.
+struct ClockPre {
+  double a, b, c, d;
+  int n;
+  bool stations;
+};
+
+__device__ __forceinline__ double ldcg_or(const double *p, int64_t k, bool in_range) {
+  return in_range ? __ldcg(p + k) : 0.0;
+}
+
+// Row cursor of the rain table as the reference moves it, clamped to the table.
+__device__ __forceinline__ int rain_row0(const hb_instance &in, const hb_ctrl *snap) {
+  return min(max(snap->rain_index, 0), in.rain_rows - 2);
+}
+
+// Loads of the clock's roles (all threads; snap is readable):
+//  thread 0       cfl, dx and the replayed dt of the next step
+//  warp 1         rain: lane l the time and rate of row (cursor + l), and the
+//                 table's last time
+//  warp 2         boundary tables: lane l the time of row l of each table;
+//                 one-row tables' values are loaded by warp 3 (lane = class)
+__device__ __forceinline__ ClockPre clock_prefetch(const hb_instance &in, const hb_ctrl *snap) {
+  ClockPre p{0.0, 0.0, 0.0, 0.0, 0, in.rain_station != nullptr};
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (tid == 0) {
+    p.a = in.cfl;
+    p.b = in.dx;
+    const int64_t step = snap->step;
+    if (in.dt_replay && step < in.n_replay) {
+      p.c = __ldcg(in.dt_replay + step);
+      p.n = 1;
+    }
+  } else if (w == 1) {
+    if (in.rain_tab && in.rain_rows >= 2) {
+      const int row = rain_row0(in, snap) + lane;
+      const int64_t C = in.rain_cols;
+      const bool ok = row < in.rain_rows;
+      p.a = ldcg_or(in.rain_tab, row * C, ok);
+      p.b = ldcg_or(in.rain_tab, row * C + 1, ok);
+      p.c = __ldcg(in.rain_tab + (in.rain_rows - 1) * C);
+    }
+  } else if (w == 2) {
+    p.a = ldcg_or(in.given_depth, (int64_t)lane * in.depth_cols,
+                  in.given_depth && lane < in.depth_rows - 1);
+    p.b = ldcg_or(in.given_wl, (int64_t)lane * in.wl_cols,
+                  in.given_wl && lane < in.wl_rows - 1);
+    p.c = ldcg_or(in.given_q, (int64_t)lane * in.q_cols, in.given_q && lane < in.q_rows - 1);
+  } else if (w == 3 && lane < HB_MAX_CLASSES) {
+    p.n = in.bc_id[lane];
+    p.a = ldcg_or(in.given_depth, p.n + 1, in.given_depth && p.n + 1 < in.depth_cols);
+    p.b = ldcg_or(in.given_wl, p.n + 1, in.given_wl && p.n + 1 < in.wl_cols);
+    p.c = ldcg_or(in.given_q, 1 + 2 * p.n, in.given_q && 2 + 2 * p.n < in.q_cols);
+    p.d = ldcg_or(in.given_q, 2 + 2 * p.n, in.given_q && 2 + 2 * p.n < in.q_cols);
+  }
+  return p;
+}
+
+// timelevel() by a warp: the first row whose time is not below t, clamped to
+// the last row.  `first` holds the times of rows 0..31 (lane = row).
+__device__ __forceinline__ int warp_timelevel(double t, const double *tab, int rows, int cols,
+                                              double first) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < rows - 1; base += 32) {
+    const int r = base + lane;
+    const bool in_range = r < rows - 1;
+    const double x = base == 0 ? first : ldcg_or(tab, (int64_t)r * cols, in_range);
+    const unsigned m = __ballot_sync(0xffffffffu, !in_range || !(t > x));
+    if (m) return min(base + __ffs(m) - 1, rows - 1);
+  }
+  return max(rows - 1, 0);
+}
+
 // The clock after a step: dt of the next step from the largest wave speed SM
 // and the any-dry flag D (HC/timeControl_Kernel.cu:164-198 per cell, torch.min,
 // then HP/SWE_CUDA.py:818-831: 10x cap, export clip, t += dt), the rain rate
-// and the boundary values at the new t.  All threads of the block call it;
-// thread 0 owns the control block.  The step's clock fields are read from
-// `snap` (the control block itself, or a copy taken at the start of the
-// finalize) and the new values are written to the control block.
+// and the boundary values at the new t.  All threads of the block call it, at
+// least four warps; the step's clock fields are read from `snap` (a copy in
+// shared memory) and the new values are written to the control block.  SM and
+// D are read by thread 0 only.
 template <typename T, int NT>
-__device__ void advance_clock(const hb_instance &in, int ii, BcTable *bct, double SM, int D,
-                              const hb_ctrl *snap) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void advance_clock(const hb_instance &in, int ii, BcTable *bct,
+                                              double SM, int D, const hb_ctrl *snap,
+                                              const ClockPre &pre) {
+  static_assert(NT >= 128, "one role per warp");
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   hb_ctrl *ctrl = in.ctrl;
-  __shared__ double s_tnew;
+  __shared__ double s_tnew, s_per;
+  __shared__ int s_lvl[3], s_row;
   if (tid == 0) {
     const double dtn = snap->dt, tn = snap->t;
     // min over cells of CFL*dx/speed; the division is monotone, so dividing
     // once by the largest speed gives the same value.
     double cand = INFINITY;
-    if (SM > 0.0) cand = (double)((T)in.cfl * (T)in.dx / (T)SM);
+    if (SM > 0.0) cand = (double)((T)pre.a * (T)pre.b / (T)SM);
     if (D) cand = fmin(cand, 60.0);
     double dtnew = (cand == INFINITY) ? dtn : cand;
     const double upper = dtn * 10.0;
@@ -339,35 +424,83 @@ __device__ void advance_clock(const hb_instance &in, int ii, BcTable *bct, doubl
       ctrl->exports = snap->exports + 1;
       if (snap->halt_on_export) ctrl->halted = 1;
     }
-    const int64_t step = snap->step;
-    if (in.dt_replay && step < in.n_replay) dtnew = in.dt_replay[step];
+    if (pre.n) dtnew = pre.c;  // replayed schedule
     if (!isfinite(dtnew)) atomicOr(&ctrl->status, 1);
     const double tnew = tn + dtnew;
     ctrl->dt = dtnew;
     ctrl->t = tnew;
-    ctrl->step = step + 1;
+    ctrl->step = snap->step + 1;
     if (tnew >= snap->t_end) ctrl->halted = 1;
     s_tnew = tnew;
   }
   __syncthreads();
   const double tnew = s_tnew;
-  // boundary values of the next step, one class per thread (step-function
-  // lookup, HC/flucCal_2ndOrder_jh_improved_Kernel.cu:355-366, 441-446)
-  if (tid < HB_MAX_CLASSES) {
-    const int k = tid, id = in.bc_id[k];
-    double hb = 0, wlb = 0, qxb = 0, qyb = 0;
-    if (in.given_depth && id + 1 < in.depth_cols) {
-      const int tl = timelevel(tnew, in.given_depth, in.depth_rows, in.depth_cols);
-      hb = in.given_depth[(int64_t)tl * in.depth_cols + id + 1];
+  if (w == 1) {
+    // rain rate at tnew (HP/SWE_CUDA.py:472-495): monotone row cursor, linear
+    // interpolation, zero from the last row on
+    double rate = 0.0, per = 0.0;
+    int row = -1;
+    if (in.rain_tab && in.rain_rows >= 2 && tnew < pre.c) {
+      const int row0 = rain_row0(in, snap), rows = in.rain_rows;
+      const int64_t C = in.rain_cols;
+      // row row0 + l is the cursor's row if t lies before the next one
+      const double next = __shfl_down_sync(0xffffffffu, pre.a, 1);
+      const unsigned m = __ballot_sync(
+          0xffffffffu, lane < 31 && (row0 + lane + 2 >= rows || tnew < next));
+      double t0, t1, v0, v1;
+      if (m) {
+        const int l = __ffs(m) - 1;
+        row = row0 + l;
+        t0 = __shfl_sync(0xffffffffu, pre.a, l);
+        v0 = __shfl_sync(0xffffffffu, pre.b, l);
+        t1 = __shfl_sync(0xffffffffu, pre.a, l + 1);
+        v1 = __shfl_sync(0xffffffffu, pre.b, l + 1);
+      } else {  // more than 31 rows ahead of the cursor
+        row = row0 + 31;
+        while (row + 2 < rows && !(tnew < __ldcg(in.rain_tab + (row + 1) * C))) row++;
+        t0 = __ldcg(in.rain_tab + row * C);
+        v0 = __ldcg(in.rain_tab + row * C + 1);
+        t1 = __ldcg(in.rain_tab + (row + 1) * C);
+        v1 = __ldcg(in.rain_tab + (row + 1) * C + 1);
+      }
+      per = (tnew - t0) / (t1 - t0);
+      rate = (v0 + per * (v1 - v0)) * snap->rain_mult;
     }
-    if (in.given_wl && id + 1 < in.wl_cols) {
-      const int tl = timelevel(tnew, in.given_wl, in.wl_rows, in.wl_cols);
-      wlb = in.given_wl[(int64_t)tl * in.wl_cols + id + 1];
+    if (lane == 0) {
+      ctrl->rain_rate = rate;
+      if (row >= 0) ctrl->rain_index = row;
+      s_row = row;
+      s_per = per;
     }
-    if (in.given_q && 2 + 2 * id < in.q_cols) {
-      const int tl = timelevel(tnew, in.given_q, in.q_rows, in.q_cols);
-      qxb = in.given_q[(int64_t)tl * in.q_cols + 1 + 2 * id];
-      qyb = in.given_q[(int64_t)tl * in.q_cols + 2 + 2 * id];
+  } else if (w == 2) {
+    // rows of the boundary tables (step-function lookup,
+    // HC/flucCal_2ndOrder_jh_improved_Kernel.cu:355-366)
+    const int ld = warp_timelevel(tnew, in.given_depth, in.given_depth ? in.depth_rows : 1,
+                                  in.depth_cols, pre.a);
+    const int lw = warp_timelevel(tnew, in.given_wl, in.given_wl ? in.wl_rows : 1, in.wl_cols,
+                                  pre.b);
+    const int lq = warp_timelevel(tnew, in.given_q, in.given_q ? in.q_rows : 1, in.q_cols, pre.c);
+    if (lane == 0) {
+      s_lvl[0] = ld;
+      s_lvl[1] = lw;
+      s_lvl[2] = lq;
+    }
+  }
+  __syncthreads();
+  if (w == 3 && lane < HB_MAX_CLASSES) {
+    // boundary values of the next step, one class per lane; row 0's values are
+    // at hand (HC/flucCal_2ndOrder_jh_improved_Kernel.cu:441-446)
+    const int k = lane, id = pre.n;
+    double hb = pre.a, wlb = pre.b, qxb = pre.c, qyb = pre.d;
+    if (s_lvl[0] > 0)
+      hb = ldcg_or(in.given_depth, (int64_t)s_lvl[0] * in.depth_cols + id + 1,
+                   id + 1 < in.depth_cols);
+    if (s_lvl[1] > 0)
+      wlb = ldcg_or(in.given_wl, (int64_t)s_lvl[1] * in.wl_cols + id + 1, id + 1 < in.wl_cols);
+    if (s_lvl[2] > 0) {
+      const int64_t q0 = (int64_t)s_lvl[2] * in.q_cols;
+      qxb = ldcg_or(in.given_q, q0 + 1 + 2 * id, 2 + 2 * id < in.q_cols);
+      qyb = ldcg_or(in.given_q, q0 + 2 + 2 * id, 2 + 2 * id < in.q_cols);
     }
     bct[ii].v[k][0] = hb;
     bct[ii].v[k][1] = wlb;
@@ -377,24 +510,27 @@ __device__ void advance_clock(const hb_instance &in, int ii, BcTable *bct, doubl
     ctrl->bc_vals[k][1] = (float)wlb;
     ctrl->bc_vals[k][2] = (float)qxb;
     ctrl->bc_vals[k][3] = (float)qyb;
-  } else if (tid == 32) {
-    ctrl->rain_rate = rain_rate_at(in, snap, ctrl, tnew);
   }
-  if (in.rain_station) {
-    __syncthreads();  // the rain cursor
-    station_rates_at(in, ctrl, tnew, tid, NT);
+  if (pre.stations) {
+    // rates of every rain station at tnew (HP/SWE_CUDA.py:472-502)
+    const int64_t C = in.rain_cols;
+    const double *r0 = s_row >= 0 ? in.rain_tab + s_row * C : nullptr;
+    for (int k = tid; k < in.n_stations; k += NT) {
+      double rate = 0.0;
+      if (r0 && k + 1 < C)
+        rate = (r0[k + 1] + s_per * (r0[C + k + 1] - r0[k + 1])) * snap->rain_mult;
+      in.station_rate[k] = rate;
+    }
   }
 }
 
-// Last tile of an instance: reduce the per-tile partials (FP64 volume and
-// outflow, largest wave speed, any dry cell), account the step's volumes,
-// flip the state buffer and advance the clock -- or, with external_dt,
-// leave the clock to hb_fused_finish and publish the speed and dry flag.
 // Sum of partials within a block, in a fixed order (lanes by a butterfly,
-// then warps in index order): the result is in thread 0.
+// then warps in index order); every thread that reads the sums (block_sum)
+// after this gets the same values.
 template <int NT>
-__device__ TilePartial block_partial_sum(double v, double o, double sm, int dry,
-                                         double (*red_d)[NT / 32], double *red_s, int *red_i) {
+__device__ __forceinline__ void block_partial_sum(double v, double o, double sm, int dry,
+                                                  double (*red_d)[NT / 32], double *red_s,
+                                                  int *red_i) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   v = warp_sum(v);
   o = warp_sum(o);
@@ -407,109 +543,132 @@ __device__ TilePartial block_partial_sum(double v, double o, double sm, int dry,
     red_i[wid] = dry;
   }
   __syncthreads();
+}
+template <int NT>
+__device__ __forceinline__ TilePartial block_sum(double (*red_d)[NT / 32], const double *red_s,
+                                                 const int *red_i) {
   TilePartial p;
   p.volume = p.outflow = p.smax = 0.0;
   p.any_dry = 0;
   p.pad = 0;
-  if (tid == 0) {
-    for (int w = 0; w < NT / 32; w++) {
-      p.volume += red_d[0][w];
-      p.outflow += red_d[1][w];
-      p.smax = fmax(p.smax, red_s[w]);
-      p.any_dry |= red_i[w];
-    }
+  for (int w = 0; w < NT / 32; w++) {
+    p.volume += red_d[0][w];
+    p.outflow += red_d[1][w];
+    p.smax = fmax(p.smax, red_s[w]);
+    p.any_dry |= red_i[w];
   }
   return p;
+}
+
+// A partial as two 16-byte loads that bypass L1.
+__device__ __forceinline__ void add_partial(const TilePartial *p, double &v, double &o,
+                                            double &sm, int &dry) {
+  const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
+  const double2 b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+  sm = fmax(sm, a.x);
+  v += a.y;
+  o += b.x;
+  dry |= (int)(__double_as_longlong(b.y) & 0xffffffffll);
 }
 
 // The instance's step is complete: reduce its `np` partials (per tile, or
 // per group of tiles), account the step's volumes, flip the state buffer
 // and advance the clock -- or, with external_dt, leave the clock to
-// hb_fused_finish and publish the speed and dry flag.  The control block is
-// copied to shared memory first (one load per thread) so that the clock
-// logic does not wait on a chain of dependent global loads.
+// hb_fused_finish and publish the speed and dry flag.  The counter that
+// elected this block was read with acquire order and every load here bypasses
+// L1, so no further fence is needed.
 template <typename T, int NT>
-__device__ void finalize_instance(const hb_instance &in, int ii, const TilePartial *parts,
-                                  int np, BcTable *bct, double (*red_d)[NT / 32], double *red_s,
-                                  int *red_i) {
+__device__ __forceinline__ void finalize_instance(const hb_instance &in, int ii,
+                                                  const TilePartial *parts, int np, BcTable *bct,
+                                                  double (*red_d)[NT / 32], double *red_s,
+                                                  int *red_i) {
   static_assert(sizeof(hb_ctrl) % 8 == 0 && sizeof(hb_ctrl) / 8 <= NT, "control block copy");
   const int tid = threadIdx.x;
   hb_ctrl *ctrl = in.ctrl;
   __shared__ hb_ctrl s_snap;
-  __threadfence();
   if (tid < (int)(sizeof(hb_ctrl) / 8))
     reinterpret_cast<unsigned long long *>(&s_snap)[tid] =
         __ldcg(reinterpret_cast<const unsigned long long *>(ctrl) + tid);
   double v = 0, o = 0, sm = 0;
   int dry = 0;
-  for (int k = tid; k < np; k += NT) {
-    const TilePartial *pp = parts + k;
-    v += __ldcg(&pp->volume);
-    o += __ldcg(&pp->outflow);
-    sm = fmax(sm, __ldcg(&pp->smax));
-    dry |= __ldcg(&pp->any_dry);
-  }
-  const TilePartial P = block_partial_sum<NT>(v, o, sm, dry, red_d, red_s, red_i);
-  __shared__ double s_sm;
-  __shared__ int s_dry, s_ext;
-  if (tid == 0) {
+#pragma unroll 4
+  for (int k = tid; k < np; k += NT) add_partial(parts + k, v, o, sm, dry);
+  __syncthreads();  // the copy of the control block
+  const ClockPre pre = clock_prefetch(in, &s_snap);
+  block_partial_sum<NT>(v, o, sm, dry, red_d, red_s, red_i);
+  if (tid == NT - 1) {  // beside the clock (thread 0)
+    const TilePartial P = block_sum<NT>(red_d, red_s, red_i);
     const hb_ctrl &c = s_snap;
-    const double V = P.volume, O = P.outflow, SM = P.smax;
-    const int D = P.any_dry;
+    const double V = P.volume, O = P.outflow;
     const double dtn = c.dt, dxd = in.dx;
     if (!isfinite(V)) atomicOr(&ctrl->status, 4);  // a NaN / inf depth somewhere in the raster
     ctrl->volume = V * dxd * dxd;
     ctrl->outflow_volume = c.outflow_volume + O * dtn * dxd;
-    if (in.rain_station) {
+    if (pre.stations) {
       double rv = 0.0;
-      for (int k = 0; k < in.n_stations; k++) rv += in.station_rate[k] * in.station_cells[k];
+      for (int k = 0; k < in.n_stations; k++)
+        rv += __ldcg(in.station_rate + k) * in.station_cells[k];
       ctrl->rain_volume = c.rain_volume + rv * dtn * dxd * dxd;
     } else {
       ctrl->rain_volume = c.rain_volume + c.rain_rate * dtn * dxd * dxd * (double)in.n_valid;
     }
     ctrl->cur = 1 - c.cur;
-    s_ext = c.external_dt;
-    if (s_ext) {
-      ctrl->ext[0] = SM;
-      ctrl->ext[1] = D ? 1.0 : 0.0;
+    if (c.external_dt) {
+      ctrl->ext[0] = P.smax;
+      ctrl->ext[1] = P.any_dry ? 1.0 : 0.0;
     }
-    s_sm = SM;
-    s_dry = D;
+    ctrl->tiles_done = 0u;
   }
-  __syncthreads();
-  if (!s_ext) advance_clock<T, NT>(in, ii, bct, s_sm, s_dry, &s_snap);
-  if (tid == 0) ctrl->tiles_done = 0u;
+  if (!s_snap.external_dt) {
+    double SM = 0.0;
+    int D = 0;
+    if (tid == 0) {
+      const TilePartial P = block_sum<NT>(red_d, red_s, red_i);
+      SM = P.smax;
+      D = P.any_dry;
+    }
+    advance_clock<T, NT>(in, ii, bct, SM, D, &s_snap, pre);
+  }
 }
 
-// The last tile of a group to finish: sum the group's `n` tile partials
-// (one per thread), store the group sum and count the group; the
-// instance's last group finalizes the step from the group sums.
+// Tiles an instance's step sums in one level; larger instances sum groups of
+// kGroupTiles first.
+constexpr int kOneGroupTiles = 4 * kGroupTiles;
+__device__ __forceinline__ int group_tiles(int n_inst_tiles) {
+  return n_inst_tiles <= kOneGroupTiles ? kOneGroupTiles : kGroupTiles;
+}
+
+// The last tile of a group to finish: an instance of one group is finalized
+// from its tile partials; otherwise sum the group's `n` tile partials (one
+// per thread), store the group sum and count the group; the instance's last
+// group finalizes the step from the group sums.
 template <typename T, int NT>
-__device__ void close_group(const hb_instance &in, int ii, const TilePartial *tiles, int n,
-                            TilePartial *gparts, unsigned *gcount, int gi, int gbase, int ng,
-                            BcTable *bct, double (*red_d)[NT / 32], double *red_s, int *red_i,
-                            int *flag) {
+__device__ __noinline__ void close_group(const hb_instance &in, int ii,
+                                            const TilePartial *tiles, int n, TilePartial *gparts,
+                                            unsigned *gcount, int gi, int gbase, int ng,
+                                            BcTable *bct, double (*red_d)[NT / 32],
+                                            double *red_s, int *red_i, int *flag) {
   static_assert(kGroupTiles <= NT, "one tile partial per thread");
   const int tid = threadIdx.x;
-  __threadfence();
-  double v = 0, o = 0, sm = 0;
-  int dry = 0;
-  if (tid < n) {
-    const TilePartial *pp = tiles + tid;
-    v = __ldcg(&pp->volume);
-    o = __ldcg(&pp->outflow);
-    sm = __ldcg(&pp->smax);
-    dry = __ldcg(&pp->any_dry);
+  if (tid == 0) gcount[gi] = 0u;  // every tile has counted: ready for the next step
+  const TilePartial *parts = tiles;
+  int np = n;
+  if (ng > 1) {
+    double v = 0, o = 0, sm = 0;
+    int dry = 0;
+    if (tid < n) add_partial(tiles + tid, v, o, sm, dry);
+    block_partial_sum<NT>(v, o, sm, dry, red_d, red_s, red_i);
+    if (tid == 0) {
+      gparts[gi] = block_sum<NT>(red_d, red_s, red_i);
+      cuda::atomic_ref<unsigned, cuda::thread_scope_device> done(in.ctrl->tiles_done);
+      *flag = (done.fetch_add(1u, cuda::memory_order_acq_rel) == (unsigned)(ng - 1));
+    }
+    __syncthreads();
+    if (!*flag) return;
+    parts = gparts + gbase;
+    np = ng;
   }
-  const TilePartial P = block_partial_sum<NT>(v, o, sm, dry, red_d, red_s, red_i);
-  if (tid == 0) {
-    gparts[gi] = P;
-    gcount[gi] = 0u;  // every tile of the group has counted: ready for the next step
-    cuda::atomic_ref<unsigned, cuda::thread_scope_device> done(in.ctrl->tiles_done);
-    *flag = (done.fetch_add(1u, cuda::memory_order_acq_rel) == (unsigned)(ng - 1));
-  }
-  __syncthreads();
-  if (*flag) finalize_instance<T, NT>(in, ii, gparts + gbase, ng, bct, red_d, red_s, red_i);
+  finalize_instance<T, NT>(in, ii, parts, np, bct, red_d, red_s, red_i);
 }
 
 // hb_fused_finish: one block per instance advances the clock from the
@@ -534,7 +693,13 @@ finish_kernel(const hb_instance *__restrict__ insts, BcTable *__restrict__ bct,
       dry = fmax(dry, __ldcg(&insts[k].ctrl->ext[1]));
     }
   }
-  advance_clock<T, kNT>(in, blockIdx.x, bct, sm, dry != 0.0 ? 1 : 0, in.ctrl);
+  __shared__ hb_ctrl s_snap;
+  if (threadIdx.x < sizeof(hb_ctrl) / 8)
+    reinterpret_cast<unsigned long long *>(&s_snap)[threadIdx.x] =
+        __ldcg(reinterpret_cast<const unsigned long long *>(in.ctrl) + threadIdx.x);
+  __syncthreads();
+  const ClockPre pre = clock_prefetch(in, &s_snap);
+  advance_clock<T, kNT>(in, blockIdx.x, bct, sm, dry != 0.0 ? 1 : 0, &s_snap, pre);
 }
 
 // Rows of the blocks a step's CTAs take.  A tile is the unit of the caller's
@@ -1659,8 +1824,9 @@ rows_step_kernel(const hb_instance *__restrict__ insts, const int32_t *__restric
     }
     __syncthreads();
     const int n_inst_tiles = in.tiles_x * in.tiles_y;
-    const int grp = lt / kGroupTiles;
-    const int gsize = min(kGroupTiles, n_inst_tiles - grp * kGroupTiles);
+    const int gt = group_tiles(n_inst_tiles);
+    const int grp = lt / gt;
+    const int gsize = min(gt, n_inst_tiles - grp * gt);
     const int gbase = in.tile_begin / kGroupTiles + ii;
     if (tid == 0) {
       TilePartial p;
@@ -1680,9 +1846,8 @@ rows_step_kernel(const hb_instance *__restrict__ insts, const int32_t *__restric
     }
     __syncthreads();
     if (s.last)
-      close_group<T, kRowsNT>(in, ii, partials + in.tile_begin + grp * kGroupTiles, gsize,
-                              gparts, gcount, gbase + grp, gbase,
-                              (n_inst_tiles + kGroupTiles - 1) / kGroupTiles, bct, s.red_d,
+      close_group<T, kRowsNT>(in, ii, partials + in.tile_begin + grp * gt, gsize, gparts, gcount,
+                              gbase + grp, gbase, (n_inst_tiles + gt - 1) / gt, bct, s.red_d,
                               s.red_s, s.red_i, &s.last2);
     __syncthreads();
   }

@@ -1009,8 +1009,9 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
   }
   __syncthreads();
   const int n_inst_tiles = in.tiles_x * in.tiles_y * kPer;
-  const int grp = lt / kGroupTiles;
-  const int gsize = min(kGroupTiles, n_inst_tiles - grp * kGroupTiles);
+  const int gt = group_tiles(n_inst_tiles);
+  const int grp = lt / gt;
+  const int gsize = min(gt, n_inst_tiles - grp * gt);
   const int gbase = tile0 / kGroupTiles + ii;
   if (tid == 0) {
     TilePartial p;
@@ -1029,9 +1030,8 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
   }
   __syncthreads();
   if (s.last)
-    close_group<float, kRowsNT>(in, ii, partials + tile0 + grp * kGroupTiles, gsize, gparts,
-                                gcount, gbase + grp, gbase,
-                                (n_inst_tiles + kGroupTiles - 1) / kGroupTiles, bct, s.red_d,
+    close_group<float, kRowsNT>(in, ii, partials + tile0 + grp * gt, gsize, gparts, gcount,
+                                gbase + grp, gbase, (n_inst_tiles + gt - 1) / gt, bct, s.red_d,
                                 s.red_s, s.red_i, &s.last2);
   __syncthreads();
   return true;
