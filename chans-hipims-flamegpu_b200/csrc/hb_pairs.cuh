@@ -381,6 +381,9 @@ constexpr int kPW = 64;             // tile width: 32 lanes x 2 cells
 constexpr int kPSWF = kPW + 8;      // staged field row: cols -4 .. 67
 constexpr int kPSWC = kPW + 32;     // staged code row: cols -16 .. 79
 
+// stations whose rates a tile keeps in shared memory (more: read from L2)
+constexpr int kSmemStations = 64;
+
 template <int TY>
 struct PairSmem {
   static constexpr int SH = TY + 4;
@@ -394,6 +397,8 @@ struct PairSmem {
   double bc[HB_MAX_CLASSES][4];
   int bctype[HB_MAX_CLASSES];
   float manning[HB_MAX_ZONES];
+  float soil[3][HB_MAX_ZONES];  // SOURCES: ks, psi, dtheta per zone
+  float srate[kSmemStations];   // SOURCES: station rates
   float ddatum[9];
   double red_d[2][kRowsNW];
   double red_s[kRowsNW];
@@ -585,6 +590,15 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
   } else if (tid >= 64 && tid < 64 + HB_MAX_ZONES) {
     s.manning[tid - 64] = (float)in.manning[tid - 64];
   }
+  if constexpr (SOURCES) {
+    if (in.cum != nullptr && tid < HB_MAX_ZONES) {
+      s.soil[0][tid] = (float)in.ks[tid];
+      s.soil[1][tid] = (float)in.psi[tid];
+      s.soil[2][tid] = (float)in.dtheta[tid];
+    }
+    if (in.rain_station != nullptr && tid >= 64 && tid - 64 < min(in.n_stations, kSmemStations))
+      s.srate[tid - 64] = (float)__ldcg(&in.station_rate[tid - 64]);
+  }
   const int bug_y = in.bug_y, bug_x = in.bug_x;
   float datum_tile = 0.f;
   if (in.datum && !skip) {
@@ -722,6 +736,7 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
     float *hmaxg = (float *)in.h_max;
     const bool infil = SOURCES && in.cum != nullptr;
     const bool stations = SOURCES && in.rain_station != nullptr;
+    const bool few = SOURCES && in.n_stations <= kSmemStations;
     const bool fwd_tile = (y0 < HB_PAD_Y && in.halo_up[0] != nullptr) ||
                           (y0 + TY > in.rows - HB_PAD_Y && in.halo_down[0] != nullptr);
     const f2 r2 = dup(dt / dx);
@@ -730,6 +745,17 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
 
 #pragma unroll 1
     for (int i = r0; i < r_end; ++i) {
+      // the pair's station ids and infiltrated depths, loaded before the faces
+      // that hide their latency (at their use they cost two to three L2 round
+      // trips a row: 56.5 us a step of 1000 x 1413 cells with stations and soils,
+      // 52.6 with rates and soils in shared memory and these loads here)
+      unsigned ids = 0;
+      f2 cum2 = dup(0.f);
+      if constexpr (SOURCES) {
+        const size_t go = (size_t)(y0 + i + HB_PAD_Y) * P + (rx0 + HB_PAD_X);
+        if (stations) ids = __ldg(reinterpret_cast<const unsigned *>(in.rain_station + go));
+        if (infil) cum2 = *reinterpret_cast<const f2 *>((const float *)in.cum + go);
+      }
       // --- x-direction: neighbours W (col 2j-1) and E (col 2j+2)
       const int kc = V.fi(i, j0);
       float Wv[4], Ev[4];
@@ -865,8 +891,9 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
       // rain (HP/SWE_CUDA.py:549 / HC/stationPrecipitation_Kernel.cu:27)
       const size_t go = (size_t)(ry + HB_PAD_Y) * P + (rx0 + HB_PAD_X);
       if (stations) {
-        hu.x += (float)__ldcg(&in.station_rate[in.rain_station[go]]) * dt;
-        hu.y += (float)__ldcg(&in.station_rate[in.rain_station[go + 1]]) * dt;
+        const unsigned ia = ids & 0xffffu, ib = ids >> 16;
+        hu.x += (few ? s.srate[ia] : (float)__ldcg(&in.station_rate[ia])) * dt;
+        hu.y += (few ? s.srate[ib] : (float)__ldcg(&in.station_rate[ib])) * dt;
       } else {
         hu = add2(hu, dup(rdt));
       }
@@ -878,16 +905,14 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
           const bool act = c ? act1 : act0;
           const bool vc = c ? vBb : vAb;
           if (!(act && vc)) continue;
-          const uint8_t kc_ = c ? kB : kA;
+          const int zc = (c ? kB : kA) & 15;
           const float hc = c ? C.h.y : C.h.x;
-          float *cum = (float *)in.cum + go + c;
-          const int zc = kc_ & 15;
-          const float K = (float)in.ks[zc], psi = (float)in.psi[zc], dth = (float)in.dtheta[zc];
-          const float F0 = *cum;
+          const float K = s.soil[0][zc], psi = s.soil[1][zc], dth = s.soil[2][zc];
+          const float F0 = c ? cum2.y : cum2.x;
           const float a = F0 + dt * K;
           const float F1 = 0.5f * (a + sqrtf(a * a + 4.f * dt * K * (psi + hc) * dth));
           const float dF = fminf(hc, F1 - F0);
-          *cum = F0 + dF;
+          ((float *)in.cum)[go + c] = F0 + dF;
           if (c) hu.y -= dF; else hu.x -= dF;
         }
       }
