@@ -713,8 +713,19 @@ finish_kernel(const hb_instance *__restrict__ insts, BcTable *__restrict__ bct,
 // of whole tiles 8-row blocks (2 rows a warp) finish sooner although every
 // band start costs an extra row of y-faces.
 constexpr int kDividePairsTiles = 592;
+// FP64 32 x 32 tiles: 16-row blocks (4 rows a warp) put 4 CTAs on an SM and balance
+// the last wave; 8-row blocks up to one of them per CTA slot.  One 2nd-order
+// step with 8- / 16- / 32-row blocks: 100^2 (16 tiles) 13.9 / 17.6 / 25.8 us,
+// 301 x 517 (170) 24.9 / 25.2 / 32.7, 512^2 (289) 30.6 / 29.7 / 34.8, 1024^2
+// (1089) 82.6 / 68.8 / 70.4, 2048^2 (4225) 279 / 220 / 223.
+constexpr int kDivide64Tiles = 148;
+inline bool is_rows64(const hb_fused_batch *b) {  // the FP64 step kernel (hb_rows64.cuh)
+  return b->dtype == HB_F64 && b->tile_x == 32 && b->tile_y == 32 &&
+         !(b->flags & HB_FLAG_TILE_TASKS);
+}
 inline int step_rows(const hb_fused_batch *b) {
   if (b->flags & (HB_FLAG_TILE_TASKS | HB_FLAG_WHOLE_TILES)) return b->tile_y;
+  if (is_rows64(b)) return b->n_tiles <= kDivide64Tiles ? 8 : 16;
   if (b->tile_x == 64 && b->tile_y == 32 && b->n_tiles <= kDividePairsTiles) return 8;
   return b->tile_y;
 }
@@ -730,7 +741,7 @@ inline int n_blocks(const hb_fused_batch *b) {
 // TilePartial, [n_groups] TilePartial (sums of groups of kGroupTiles blocks),
 // [n_groups] unsigned group counters, [n] int32 block order (rows kernel:
 // general blocks, then all-valid blocks), [3] int32 counts, [n] uint8
-// all-valid flags, 64-wide tiles only: [n] TileEntry in the order's order,
+// all-valid flags, 64-wide tiles and FP64: [n] TileEntry in the order's order,
 // then [n_instances] BcTable, then [n_instances][kMapsPerInstance]
 // CUtensorMap.  Instance i's groups start at (its first block) / kGroupTiles
 // + i, which never overlaps instance i + 1's.
@@ -751,7 +762,7 @@ inline size_t ws_counts_offset(const hb_fused_batch *b) {
   return ws_order_offset(b) + align256((size_t)n_blocks(b) * sizeof(int32_t));
 }
 inline size_t ws_flags_offset(const hb_fused_batch *b) { return ws_counts_offset(b) + 256; }
-// What a block of the two-cells-per-lane step needs before it can issue its
+// What a block of the two-cells-per-lane or the FP64 step needs before it can issue its
 // loads, in one 16-byte record: the block (~block when it holds no valid
 // cell), its instance and that instance's control block.
 struct alignas(16) TileEntry {
@@ -763,8 +774,13 @@ static_assert(sizeof(TileEntry) == 16, "one 16-byte load per tile");
 inline size_t ws_entries_offset(const hb_fused_batch *b) {
   return ws_flags_offset(b) + align256((size_t)n_blocks(b));
 }
+// (the FP64 step on whole tiles reads the order list instead: 37 bytes of
+// workspace a tile, which keeps the fixed scratch's tile limit)
+inline bool has_entries(const hb_fused_batch *b) {
+  return b->tile_x == 64 || (is_rows64(b) && !(b->flags & HB_FLAG_WHOLE_TILES));
+}
 inline size_t ws_entries_bytes(const hb_fused_batch *b) {
-  return b->tile_x == 64 ? align256((size_t)n_blocks(b) * sizeof(TileEntry)) : 0;
+  return has_entries(b) ? align256((size_t)n_blocks(b) * sizeof(TileEntry)) : 0;
 }
 inline size_t ws_bct_offset(const hb_fused_batch *b) {
   return ws_entries_offset(b) + ws_entries_bytes(b);
@@ -1856,6 +1872,9 @@ rows_step_kernel(const hb_instance *__restrict__ insts, const int32_t *__restric
 // The FP32 2nd-order step with two cells per lane (64-wide tiles).
 #include "hb_pairs.cuh"
 
+// The FP64 step.
+#include "hb_rows64.cuh"
+
 // Prepare: rain rate and boundary values at t, counters; the volume at t is
 // summed by prepare_volume_kernel, launched after this one.
 template <typename T>
@@ -1959,7 +1978,7 @@ int launch_steps(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
 // cell is out of its reach; the rows kernel runs those tiles in its all-valid
 // build and the others in its general build.
 // ---------------------------------------------------------------------------
-template <int TY, int TW, int PER = 1>
+template <int TY, int TW, int PER = 1, bool EMPTY = (TW == 64)>
 __global__ void __launch_bounds__(kRowsNT)
 classify_tiles_kernel(const hb_instance *__restrict__ insts, const int32_t *__restrict__ tile_inst,
                       int n_tiles, uint8_t *__restrict__ flags) {
@@ -1983,8 +2002,8 @@ classify_tiles_kernel(const hb_instance *__restrict__ insts, const int32_t *__re
   }
   ok = __syncthreads_and(ok) != 0;
   own = __syncthreads_or(own) != 0;
-  // 2 (64-wide tiles only): no valid cell of its own, nothing to step
-  if (threadIdx.x == 0) flags[tile] = ok ? 1 : ((TW == kPW && !own) ? 2 : 0);
+  // 2 (64-wide tiles and FP64): no valid cell of its own, nothing to step
+  if (threadIdx.x == 0) flags[tile] = ok ? 1 : ((EMPTY && !own) ? 2 : 0);
 }
 
 // Stable partition of the tiles by flag, one block: order = general tiles
@@ -2165,12 +2184,14 @@ int launch_rows_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
 // both at once; the general build keeps the register cap of 3 CTAs per SM
 // (its ghost-face branches spill under a tighter one) and MINB caps the
 // all-valid build.
-template <int TY, bool SOURCES, int ORDER>
-int launch_mixed(const hb_fused_batch *b, int nsteps, int grid, int n_live, int n_valid_end, int n,
-                 cudaStream_t st) {
-  using S = PairSmem<TY>;
-  auto *km = pairs_mixed_kernel<TY, SOURCES, ORDER>;
-  const int rc = set_smem_attr(reinterpret_cast<const void *>(km), (int)sizeof(S));
+// One programmatic launch per step of a kernel over the prepared block list.
+struct ListCounts {
+  int n_live, n_valid_end, n;
+};
+template <typename K, typename... Extra>
+int launch_list(K *kernel, size_t smem, const hb_fused_batch *b, int nsteps, int grid,
+                const ListCounts &c, cudaStream_t st, Extra... extra) {
+  const int rc = set_smem_attr(reinterpret_cast<const void *>(kernel), (int)smem);
   if (rc) return rc;
   char *ws = reinterpret_cast<char *>(b->workspace);
   cudaLaunchAttribute at[1];
@@ -2179,49 +2200,80 @@ int launch_mixed(const hb_fused_batch *b, int nsteps, int grid, int n_live, int 
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(std::max(grid, 1));
   cfg.blockDim = dim3(kRowsNT);
-  cfg.dynamicSmemBytes = sizeof(S);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   for (int k = 0; k < nsteps; k++) {
     const cudaError_t e = cudaLaunchKernelEx(
-        &cfg, km, b->instances, reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b)),
-        n_live, n_valid_end, n, reinterpret_cast<TilePartial *>(ws),
+        &cfg, kernel, b->instances, reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b)),
+        c.n_live, c.n_valid_end, c.n, reinterpret_cast<TilePartial *>(ws),
         reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b)),
         reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b)),
         reinterpret_cast<BcTable *>(ws + ws_bct_offset(b)),
-        reinterpret_cast<const CUtensorMap *>(ws + ws_maps_offset(b)));
+        reinterpret_cast<const CUtensorMap *>(ws + ws_maps_offset(b)), extra...);
     if (e != cudaSuccess) return set_error(HB_ERR_CUDA, "hb_fused_step: %s", cudaGetErrorString(e));
   }
   return check_launch("hb_fused_step");
+}
+
+// The lengths of the prepared list, from prepare (one read-back there), so that
+// a block's first load is its own entry.
+int list_counts(const hb_fused_batch *b, ListCounts &c) {
+  std::lock_guard<std::mutex> lock(g_side_mu);
+  const auto it = g_general_tiles.find(b->workspace);
+  if (it == g_general_tiles.end())
+    return set_error(HB_ERR_ARG, "hb_fused_step: run hb_fused_prepare on this workspace first");
+  c.n = n_blocks(b);
+  const int n_general = std::min(std::max(it->second.general, 0), c.n);
+  const int n_empty = std::min(std::max(it->second.empty, 0), n_general);
+  c.n_live = n_general - n_empty;
+  c.n_valid_end = c.n_live + c.n - n_general;
+  return HB_OK;
+}
+
+template <int TY, bool SOURCES, int ORDER>
+int launch_rows64_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
+  ListCounts c{};
+  const int rc = list_counts(b, c);
+  if (rc) return rc;
+  const int32_t *order = reinterpret_cast<const int32_t *>(
+      reinterpret_cast<char *>(b->workspace) + ws_order_offset(b));
+  return launch_list(rows64_kernel<TY, SOURCES, ORDER>, sizeof(Rows64Smem<TY>), b, nsteps,
+                     b->grid_blocks > 0 ? std::min(b->grid_blocks, c.n) : c.n, c, st,
+                     has_entries(b) ? nullptr : order, b->tile_instance);
+}
+template <int ORDER>
+int launch_rows64(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
+  const bool src = (b->flags & HB_FLAG_SOURCES) != 0;
+  switch (step_rows(b)) {
+    case 8:
+      return src ? launch_rows64_impl<8, true, ORDER>(b, nsteps, st)
+                 : launch_rows64_impl<8, false, ORDER>(b, nsteps, st);
+    case 16:
+      return src ? launch_rows64_impl<16, true, ORDER>(b, nsteps, st)
+                 : launch_rows64_impl<16, false, ORDER>(b, nsteps, st);
+    default:
+      return src ? launch_rows64_impl<32, true, ORDER>(b, nsteps, st)
+                 : launch_rows64_impl<32, false, ORDER>(b, nsteps, st);
+  }
 }
 
 template <int MINB, bool SOURCES, int ORDER = 2>
 int launch_pairs_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   constexpr int TY = 32;
   using S = PairSmem<TY>;
-  const int n = n_blocks(b);
-  // the list lengths come from prepare (one read-back there), so that a
-  // block's first load is its own entry
-  // entries: general blocks with a valid cell [0, n_live), all-valid blocks
-  // [n_live, n_live + n_valid), blocks without a valid cell [.., n)
-  int n_general = 0, n_empty = 0;
-  {
-    std::lock_guard<std::mutex> lock(g_side_mu);
-    const auto it = g_general_tiles.find(b->workspace);
-    if (it == g_general_tiles.end())
-      return set_error(HB_ERR_ARG, "hb_fused_step: run hb_fused_prepare on this workspace first");
-    n_general = std::min(std::max(it->second.general, 0), n);
-    n_empty = std::min(std::max(it->second.empty, 0), n_general);
-  }
-  const int n_valid = n - n_general, n_live = n_general - n_empty;
+  ListCounts c{};
+  const int lc = list_counts(b, c);
+  if (lc) return lc;
+  const int n = c.n, n_live = c.n_live, n_valid = c.n_valid_end - c.n_live;
+  const int n_general = n - n_valid;
   // 8-row blocks (a small batch): one launch whatever the register cap asked for
   if (step_rows(b) == 8)
-    return launch_mixed<8, SOURCES, ORDER>(
-        b, nsteps, b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : n, n_live, n_live + n_valid,
-        n, st);
+    return launch_list(pairs_mixed_kernel<8, SOURCES, ORDER>, sizeof(PairSmem<8>), b, nsteps,
+                       b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : n, c, st);
   if (MINB == 4 && b->grid_blocks <= 0)
-    return launch_mixed<TY, SOURCES, ORDER>(b, nsteps, n, n_live, n_live + n_valid, n, st);
+    return launch_list(pairs_mixed_kernel<TY, SOURCES, ORDER>, sizeof(S), b, nsteps, n, c, st);
   char *ws = reinterpret_cast<char *>(b->workspace);
   TilePartial *parts = reinterpret_cast<TilePartial *>(ws);
   TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b));
@@ -2442,6 +2494,15 @@ int prepare_impl(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_map
     else if (b->tile_x == kPW)
       classify_tiles_kernel<32, kPW><<<b->n_tiles, kRowsNT, 0, st>>>(
           b->instances, b->tile_instance, b->n_tiles, flags);
+    else if (is_rows64(b) && per == 4)
+      classify_tiles_kernel<8, kTW, 4, true><<<n, kRowsNT, 0, st>>>(b->instances,
+                                                                    b->tile_instance, n, flags);
+    else if (is_rows64(b) && per == 2)
+      classify_tiles_kernel<16, kTW, 2, true><<<n, kRowsNT, 0, st>>>(b->instances,
+                                                                     b->tile_instance, n, flags);
+    else if (is_rows64(b))
+      classify_tiles_kernel<32, kTW, 1, true><<<n, kRowsNT, 0, st>>>(b->instances,
+                                                                     b->tile_instance, n, flags);
     else if (b->tile_y == 64)
       classify_tiles_kernel<64, kTW><<<b->n_tiles, kRowsNT, 0, st>>>(
           b->instances, b->tile_instance, b->n_tiles, flags);
@@ -2451,7 +2512,7 @@ int prepare_impl(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_map
     order_tiles_kernel<<<1, kOrderNT, 0, st>>>(
         flags, n, reinterpret_cast<int32_t *>(ws + ws_order_offset(b)),
         reinterpret_cast<int32_t *>(ws + ws_counts_offset(b)));
-    if (b->tile_x == kPW)
+    if (has_entries(b))
       tile_entries_kernel<<<(n + 255) / 256, 256, 0, st>>>(
           reinterpret_cast<const int32_t *>(ws + ws_order_offset(b)), n, per, b->tile_instance,
           b->instances, reinterpret_cast<TileEntry *>(ws + ws_entries_offset(b)));
@@ -2528,8 +2589,7 @@ extern "C" int hb_fused_step(const hb_fused_batch *b, int nsteps, void *stream) 
       if (minb == 0) return launch_rows<float, 32, true, 1, 1>(b, nsteps, st);
       if (minb == 5) return launch_rows<float, 32, true, 5, 1>(b, nsteps, st);
     }
-    if (tx == kTW && ty == 32 && b->dtype == HB_F64)
-      return launch_rows<double, 32, false, 1, 1>(b, nsteps, st);
+    if (is_rows64(b)) return launch_rows64<1>(b, nsteps, st);
     return set_error(HB_ERR_ARG, "hb_fused_step: order 1 is built for FP32 64 x 32 tiles (minb "
                                  "0 or 4) and 32 x 32 tiles (minb 0 or 5), and FP64 32 x 32 tiles");
   }
@@ -2551,7 +2611,7 @@ extern "C" int hb_fused_step(const hb_fused_batch *b, int nsteps, void *stream) 
       if (ty == 64 && minb == 0) return launch_rows<float, 64>(b, nsteps, st);
       if (ty == 64 && minb == 4) return launch_rows<float, 64, true, 4>(b, nsteps, st);
     } else if (b->dtype == HB_F64) {
-      if (ty == 32) return launch_rows<double, 32>(b, nsteps, st);
+      if (is_rows64(b)) return launch_rows64<2>(b, nsteps, st);
     }
     return set_error(HB_ERR_ARG, "hb_fused_step: rows kernel %dx%d not built for this dtype", ty, tx);
   }

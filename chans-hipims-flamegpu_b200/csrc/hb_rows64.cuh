@@ -1,0 +1,665 @@
+// hb_rows64.cuh -- the FP64 step kernel.
+//
+// Included by hb_fused.cu inside its anonymous namespace (TilePartial, BcTable,
+// close_group, mbarrier/TMA helpers, TileEntry).  Same scheme, decisions and
+// data layout as the FP32 kernels (HC/flucCal_2ndOrder_jh_improved_Kernel.cu:43-506,
+// HC/fluxCal_jh_modified_surface_Kernel.cu:96-139, 577-610 per face,
+// HC/friction_implicit_andUpdate_jh_Kernel.cu:22-146 and
+// HC/timeControl_Kernel.cu:164-198 per cell, HC/fluxMaskGenerator_Kernel.cu:19-42
+// for the activity rule).
+//
+// What bounds it: FP64 issue.  An SM starts 64 FP64 lanes a cycle, and a cell
+// needs about 400 FP64 operations (two faces, eight slopes, one update), so the
+// design spends as few of them as it can and keeps 16 warps an SM to cover
+// their latency:
+//  * a CTA of 4 warps owns 32 columns x TY rows staged by TMA, lane = column,
+//    each warp walks TY/4 rows; every face is evaluated once (south faces are
+//    kept for the next row, west faces go to the west lane by shuffle, the
+//    faces east of lane 31 are evaluated by the first lanes of the same warp
+//    before the walk, one row a lane, so no warp waits for another);
+//  * reciprocals and square roots by one table-free cubic step from the
+//    hardware's approximate seed (rcp64, sqrt64: 3 and 6 FP64 operations
+//    instead of a division of about twelve and a root of about ten), one
+//    reciprocal per edge for both velocities, one for the wave span, dt / dx once
+//    per tile; the contact speed's sign is read off numerator and denominator;
+//  * a missing neighbour is replaced by its ghost state before the face, so
+//    ghost faces go through the same code as interior ones and cost selects
+//    instead of a second, divergent evaluation;
+//  * minmod and the dry tests of non-negative values compare on the integer
+//    pipe where that is exact.
+// Measured (B200, 2nd order, steps back to back), against the FP64 build of the
+// one-cell-per-lane kernel it replaced (IEEE divisions, pow, 191-230
+// registers, two launches): 1024^2 282 -> 68 us a step, 2048^2 960 -> 220 us,
+// 301 x 517 in 1st order 77 -> 22 us.  1024^2: 41 M warp instructions (81 M
+// before), 15 M of them FP64; issue active 54 %, FP64 pipe 40 %, 16 warps an SM.
+// Error against 64-bit references of the same steps: unchanged (1.1e-13 of the
+// discharge's norm after 8 steps, set by the reference's friction form).
+// Every operation is pinned (__dadd_rn, __dmul_rn, __fma_rn), so a face
+// evaluated by two tiles, or by the general and the all-valid path, comes out
+// bit for bit the same.
+
+__device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sb(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double mu(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// 1 / x for normal x: the hardware's seed r0 (relative error e; 2^-19.9 at most
+// over 6e7 values of 2^-60..2^40) and the third-order iteration
+// r0 (1 + e + e^2) (Householder's method for 1/r - x), remainder e^3.  Largest
+// error over those values 2^-53 of the result.
+__device__ __forceinline__ double rcp64(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fm(-x, r, 1.0);
+  return fm(r, fm(e, e, e), r);
+}
+// sqrt(x) for x = 0 or normal x > 0: y0 ~ 1/sqrt(x) from the hardware, s0 = x y0,
+// e = 1 - s0 y0, and sqrt(x) = s0 (1 - e)^(-1/2) by its binomial series to e^2
+// (remainder 5/16 e^3).  Largest error over the same values 2^-52 of the result.
+__device__ __forceinline__ double sqrt64(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double s0 = mu(x, y);
+  const double e = fm(-s0, y, 1.0);
+  const double s = fm(mu(s0, e), fm(0.375, e, 0.5), s0);
+  return x > 0.0 ? s : 0.0;
+}
+__device__ __forceinline__ double max64(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ double min64(double a, double b) { return a < b ? a : b; }
+// max(x, 0) by the sign bit
+__device__ __forceinline__ double pos64(double x) { return __double2hiint(x) < 0 ? 0.0 : x; }
+__device__ __forceinline__ double abs64(double x) { return fabs(x); }
+// minmod(x, y) (HC/flucCal_2ndOrder_jh_improved_Kernel.cu:74-81): the sign test
+// on the sign bits (a zero argument has the smaller magnitude and is selected)
+__device__ __forceinline__ double mm64(double x, double y) {
+  const double m = fabs(x) < fabs(y) ? x : y;
+  return (__double2hiint(x) ^ __double2hiint(y)) < 0 ? 0.0 : m;
+}
+
+struct Cel64 {
+  double h, qx, qy, z;
+};
+// fluxes in the global frame from the minus (west / south) side, bed-slope
+// terms of both sides
+struct Fc64 {
+  double fh, fx, fy, sa, sb;
+};
+
+// One face in its own frame from the cells' depths and beds (A minus, B plus)
+// and the edge states L, R (depth, bed, normal and tangential discharge).
+template <int ORDER>
+__device__ __forceinline__ void face_core64(double Ah, double Az, double Bh, double Bz,
+                                            double Lh, double Lz, double Lqn, double Lqt,
+                                            double Rh, double Rz, double Rqn, double Rqt,
+                                            double &fh, double &fn, double &ft, double &sa,
+                                            double &sbt) {
+  const double hs = kHSmall, g = kG;
+  const bool dryA = Ah < hs, dryB = Bh < hs;
+  // velocities of the edge states before the hydrostatic step; a dry cell's
+  // edge carries none
+  const double il = (dryA || Lh < hs) ? 0.0 : rcp64(Lh);
+  const double ir = (dryB || Rh < hs) ? 0.0 : rcp64(Rh);
+  const double uL = mu(Lqn, il), vL = mu(Lqt, il), uR = mu(Rqn, ir), vR = mu(Rqt, ir);
+  // hydrostatic reconstruction
+  const double wa = ad(Az, Ah), wb = ad(Bz, Bh);
+  const bool down = wa > wb;
+  const double hi = down ? wa : wb, lo = down ? wb : wa;
+  double Lw = max64(min64(ad(Lh, Lz), hi), lo);
+  double Rw = max64(min64(ad(Rh, Rz), hi), lo);
+  if constexpr (ORDER == 2) {
+    const double m = max64(Lw, Rw);
+    Lw = down ? m : Lw;
+    Rw = down ? Rw : m;
+  } else {
+    const bool flip = mu(sb(wa, wb), sb(Lw, Rw)) < 0.0;
+    const double avg = mu(ad(Lw, Rw), 0.5);
+    Lw = flip ? avg : Lw;
+    Rw = flip ? avg : Rw;
+  }
+  const double zbm = max64(sb(Lw, Lh), sb(Rw, Rh));
+  const double hL = pos64(sb(Lw, zbm)), hR = pos64(sb(Rw, zbm));
+  sa = mu(mu(0.5 * kG, ad(Ah, hL)), sb(sb(Lw, hL), Az));
+  sbt = mu(mu(0.5 * kG, ad(Bh, hR)), sb(sb(Rw, hR), Bz));
+  // HLLC
+  const bool thinL = hL <= hs, thinR = hR <= hs;
+  const double qL = mu(uL, hL), qR = mu(uR, hR);
+  const double gL = mu(g, hL), gR = mu(g, hR);
+  const double aL = sqrt64(gL), aR = sqrt64(gR);
+  const double us = sb(fm(ad(uL, uR), 0.5, aL), aR);
+  const double as = fabs(fm(ad(aL, aR), 0.5, mu(sb(uL, uR), 0.25)));
+  const double sL = thinL ? fm(-2.0, aR, uR) : min64(sb(uL, aL), sb(us, as));
+  const double sR = thinR ? fm(2.0, aL, uL) : max64(ad(uR, aR), ad(us, as));
+  const double nL = fm(uL, qL, mu(mu(0.5, gL), hL)), nR = fm(uR, qR, mu(mu(0.5, gR), hR));
+  const double pL = mu(hL, sb(uL, sL)), pR = mu(hR, sb(uR, sR));
+  // contact speed sM = num / den: only its sign is needed (den = 0: neither)
+  const double num = sb(mu(sL, pR), mu(sR, pL)), den = sb(pR, pL);
+  const int sg = __double2hiint(num) ^ __double2hiint(den);
+  const bool zero = num == 0.0;
+  const bool some = den != 0.0;
+  const bool left = 0.0 <= sL;
+  const bool midL = !left && some && (sg >= 0 || zero);
+  const bool midR = !left && some && !(sg >= 0 || zero) && 0.0 <= sR;
+  const bool mid = midL || midR;
+  const double inv = rcp64(sb(sR, sL)), sLR = mu(sL, sR);
+  const double hM = mu(fm(sLR, sb(hR, hL), sb(mu(sR, qL), mu(sL, qR))), inv);
+  const double nM = mu(fm(sLR, sb(qR, qL), sb(mu(sR, nL), mu(sL, nR))), inv);
+  const bool none = hL < hs && hR < hs;
+  const bool dd = dryA && dryB;
+  fh = left ? qL : (mid ? hM : qR);
+  fn = left ? nL : (mid ? nM : nR);
+  if (none || dd) fh = fn = 0.0;
+  // the tangential flux is the mass flux times the upwind tangential velocity
+  ft = mu(fh, (left || midL) ? vL : vR);
+  if (dd) sa = sbt = 0.0;
+}
+
+// Ghost of cell C across a missing neighbour along DIR
+// (HC/flucCal_2ndOrder_jh_improved_Kernel.cu:197-332; FALL, type 9:
+// HC/fluxCal_jh_modified_surface_Kernel.cu:389-396).  False: no ghost rule.
+template <int DIR, int ORDER>
+__device__ __forceinline__ bool ghost64(int type, const double *bc, const Cel64 &C, Cel64 &G) {
+  G = C;
+  switch (type) {
+    case 3:  // both components change sign on x-faces, neither on y-faces
+      if (DIR == 0) {
+        G.qx = -C.qx;
+        G.qy = -C.qy;
+      }
+      return true;
+    case 4:
+      if (DIR == 0) G.qx = -C.qx; else G.qy = -C.qy;
+      return true;
+    case 5:
+      return true;
+    case 6:
+      G.h = bc[0];
+      return true;
+    case 7:
+      G.qx = bc[2];
+      G.qy = bc[3];
+      return true;
+    case 8:
+      G.h = sb(max64(bc[1], C.z), C.z);
+      return true;
+    case 9:
+      if (ORDER != 1) return false;
+      G.h = G.qx = G.qy = 0.0;
+      return true;
+    default:
+      return false;
+  }
+}
+
+template <int TY>
+struct Rows64Smem {
+  static constexpr int SH = TY + 4;
+  double f[4][SH * kSWF];  // h, qx, qy, z
+  double hmax[TY * kTW];
+  uint8_t code[SH * kSWC];
+  alignas(8) unsigned long long bar;
+  double xe[TY][4];   // face between cols 31 | 32: fh, fx, fy, sa
+  double sxw[TY][4];  // x-slope of col -1: h, qx, qy, z
+  double bc[HB_MAX_CLASSES][4];
+  int bctype[HB_MAX_CLASSES];
+  double manning[HB_MAX_ZONES];
+  double red_d[2][kRowsNW];
+  double red_s[kRowsNW];
+  int red_i[kRowsNW];
+  int last, last2;
+  static constexpr unsigned kTxBytes =
+      (unsigned)(4 * SH * kSWF * sizeof(double) + TY * kTW * sizeof(double) + SH * kSWC);
+};
+
+template <int TY>
+struct View64 {
+  const Rows64Smem<TY> &s;
+  __device__ __forceinline__ int fi(int i, int j) const { return (i + 2) * kSWF + (j + 4); }
+  __device__ __forceinline__ Cel64 cell(int i, int j) const {
+    const int k = fi(i, j);
+    return Cel64{s.f[0][k], s.f[1][k], s.f[2][k], s.f[3][k]};
+  }
+  __device__ __forceinline__ uint8_t code(int i, int j) const {
+    return s.code[(i + 2) * kSWC + (j + 16)];
+  }
+};
+
+// Slopes of c between its minus-side neighbour m and plus-side neighbour p (a
+// missing one is replaced by c, HC/flucCal_2ndOrder_jh_improved_Kernel.cu:416-428);
+// ORDER 1 uses the bed's only.
+template <int ORDER, bool ALLV>
+__device__ __forceinline__ Cel64 slope64(const Cel64 &c, const Cel64 &m, bool vm, const Cel64 &p,
+                                         bool vp) {
+  auto one = [&](double x, double a, double b) {
+    const double lo = ALLV || vm ? a : x, up = ALLV || vp ? b : x;
+    return mm64(sb(x, lo), sb(up, x));
+  };
+  Cel64 s{0.0, 0.0, 0.0, one(c.z, m.z, p.z)};
+  if constexpr (ORDER == 2) {
+    s.h = one(c.h, m.h, p.h);
+    s.qx = one(c.qx, m.qx, p.qx);
+    s.qy = one(c.qy, m.qy, p.qy);
+  }
+  return s;
+}
+
+// Face between A (minus side, code ca) and B (plus side, code cb) along DIR
+// from the cells and their slopes; general tiles: a missing side becomes the
+// other cell's ghost, without reconstruction.
+template <int DIR, int ORDER, bool ALLV, int TY>
+__device__ __forceinline__ Fc64 face64(const Rows64Smem<TY> &s, Cel64 A, uint8_t ca, Cel64 B,
+                                       uint8_t cb, Cel64 sA, Cel64 sB) {
+  bool va = true, vb = true, rule = true;
+  if constexpr (!ALLV) {
+    va = is_valid(ca);
+    vb = is_valid(cb);
+    if (va != vb) {
+      const int cls = (va ? ca : cb) >> 4;
+      Cel64 G;
+      rule = ghost64<DIR, ORDER>(s.bctype[cls], s.bc[cls], va ? A : B, G);
+      if (va) B = G; else A = G;
+      sA = sB = Cel64{0.0, 0.0, 0.0, 0.0};
+    }
+  }
+  Cel64 L, R;
+  if constexpr (ORDER == 2) {
+    L = Cel64{fm(0.5, sA.h, A.h), fm(0.5, sA.qx, A.qx), fm(0.5, sA.qy, A.qy), fm(0.5, sA.z, A.z)};
+    R = Cel64{fm(-0.5, sB.h, B.h), fm(-0.5, sB.qx, B.qx), fm(-0.5, sB.qy, B.qy),
+              fm(-0.5, sB.z, B.z)};
+  } else {
+    // the bed alone takes half its slope, on a side whose neighbour is wet
+    L = A;
+    R = B;
+    if (B.h > kHSmall) L.z = fm(0.5, sA.z, A.z);
+    if (A.h > kHSmall) R.z = fm(-0.5, sB.z, B.z);
+  }
+  Fc64 o;
+  double fn, ft;
+  if constexpr (DIR == 0) {
+    face_core64<ORDER>(A.h, A.z, B.h, B.z, L.h, L.z, L.qx, L.qy, R.h, R.z, R.qx, R.qy, o.fh, fn,
+                       ft, o.sa, o.sb);
+    o.fx = fn;
+    o.fy = ft;
+  } else {
+    // normal +y, tangent -x; the tangential flux is linear in the tangential
+    // discharge, so +qx in gives +Fx out
+    face_core64<ORDER>(A.h, A.z, B.h, B.z, L.h, L.z, L.qy, L.qx, R.h, R.z, R.qy, R.qx, o.fh, fn,
+                       ft, o.sa, o.sb);
+    o.fx = ft;
+    o.fy = fn;
+  }
+  if constexpr (!ALLV) {
+    if (!(va || vb) || !rule) o = Fc64{0.0, 0.0, 0.0, 0.0, 0.0};
+    if (!va) o.sa = 0.0;
+    if (!vb) o.sb = 0.0;
+  }
+  return o;
+}
+
+// One block of TY rows of a step (tile or part of a tile); returns false when
+// its data did not arrive within the bounded wait.
+template <int TY, bool SOURCES, bool ALLV, int ORDER>
+__device__ __forceinline__ bool rows64_tile(Rows64Smem<TY> &s, unsigned &phase, const TileEntry en,
+                                            const hb_instance *__restrict__ insts,
+                                            TilePartial *__restrict__ partials,
+                                            TilePartial *__restrict__ gparts,
+                                            unsigned *__restrict__ gcount,
+                                            BcTable *__restrict__ bct,
+                                            const CUtensorMap *__restrict__ maps) {
+  using S = Rows64Smem<TY>;
+  constexpr int R = TY / kRowsNW;
+  constexpr int kPer = 32 / TY;
+  const View64<TY> V{s};
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const double hs = kHSmall, g = kG;
+  const bool skip = !ALLV && en.tile < 0;  // no valid cell: adds a zero partial
+  const int tile = en.tile < 0 ? ~en.tile : en.tile;
+  const int ii = en.inst;
+  const hb_instance &in = insts[ii];
+  hb_ctrl *ctrl = en.ctrl;
+  if (__ldcg(&ctrl->halted)) return true;
+  const int tile0 = in.tile_begin * kPer;
+  const int lt = tile - tile0;
+  const int tyi = lt / in.tiles_x, txi = lt - tyi * in.tiles_x;
+  const int y0 = tyi * TY, x0 = txi * kTW;
+  const int cur = __ldcg(&ctrl->cur);
+  const double dt = __ldcg(&ctrl->dt);
+  const bool first = __ldcg(&ctrl->t) == 0.0;
+  const double rdt = mu(__ldcg(&ctrl->rain_rate), dt);
+  const int P = in.pitch;
+  if (tid == 0 && !skip) {
+    const CUtensorMap *m = maps + (size_t)ii * kMapsPerInstance;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_expect_tx(&s.bar, S::kTxBytes);
+    tma_load_2d(s.f[0], m + 0 + cur, x0, y0, &s.bar);
+    tma_load_2d(s.f[1], m + 2 + cur, x0, y0, &s.bar);
+    tma_load_2d(s.f[2], m + 4 + cur, x0, y0, &s.bar);
+    tma_load_2d(s.f[3], m + 6, x0, y0, &s.bar);
+    tma_load_2d(s.hmax, m + 7, x0 + HB_PAD_X, y0 + HB_PAD_Y, &s.bar);
+    tma_load_2d(s.code, m + 8, x0, y0, &s.bar);
+  }
+  if (tid < HB_MAX_CLASSES) {
+    if constexpr (!ALLV) {
+      s.bctype[tid] = in.bc_type[tid];
+      for (int q = 0; q < 4; q++) s.bc[tid][q] = __ldcg(&bct[ii].v[tid][q]);
+    }
+  } else if (tid >= 64 && tid < 64 + HB_MAX_ZONES) {
+    s.manning[tid - 64] = in.manning[tid - 64];
+  }
+  const int bug_y = in.bug_y, bug_x = in.bug_x;
+  const double r = dt / in.dx;
+  if (!skip) {
+    const bool arrived = mbar_wait(&s.bar, phase, 4000000000LL);
+    if (__syncthreads_or(!arrived)) {
+      if (tid == 0) atomicOr(&ctrl->status, 2);
+      mbar_wait(&s.bar, phase, 4000000000LL);
+      return false;
+    }
+    phase ^= 1u;
+  }
+
+  double vol = 0.0, smax = 0.0, outf = 0.0;
+  int any_dry = 0;
+  if (!skip) {
+    const int j = lane, r0 = w * R;
+    auto valid = [](uint8_t k) -> bool { return ALLV || is_valid(k); };
+    // --- faces east of lane 31 and x-slopes of column -1, one row a lane
+    if (lane < R) {
+      const int i = r0 + lane;
+      const Cel64 a = V.cell(i, 31), b = V.cell(i, 32);
+      const uint8_t ca = V.code(i, 31), cb = V.code(i, 32);
+      const Cel64 sa = slope64<ORDER, ALLV>(a, V.cell(i, 30), valid(V.code(i, 30)), b, valid(cb));
+      const Cel64 sb_ = slope64<ORDER, ALLV>(b, a, valid(ca), V.cell(i, 33),
+                                             valid(V.code(i, 33)));
+      const Fc64 f = face64<0, ORDER, ALLV, TY>(s, a, ca, b, cb, sa, sb_);
+      s.xe[i][0] = f.fh;
+      s.xe[i][1] = f.fx;
+      s.xe[i][2] = f.fy;
+      s.xe[i][3] = f.sa;
+      const Cel64 m1 = slope64<ORDER, ALLV>(V.cell(i, -1), V.cell(i, -2), valid(V.code(i, -2)),
+                                            V.cell(i, 0), valid(V.code(i, 0)));
+      s.sxw[i][0] = m1.h;
+      s.sxw[i][1] = m1.qx;
+      s.sxw[i][2] = m1.qy;
+      s.sxw[i][3] = m1.z;
+    }
+    // --- column window: row r0, its y-slopes and its north face
+    Cel64 C = V.cell(r0, j), Sx = V.cell(r0 + 1, j);
+    uint8_t kC = V.code(r0, j), kS = V.code(r0 + 1, j), kN = V.code(r0 - 1, j);
+    double Nh;
+    Cel64 syC;
+    Fc64 nf;
+    {
+      const Cel64 N = V.cell(r0 - 1, j);
+      const Cel64 syN = slope64<ORDER, ALLV>(N, C, valid(kC), V.cell(r0 - 2, j),
+                                             valid(V.code(r0 - 2, j)));
+      syC = slope64<ORDER, ALLV>(C, Sx, valid(kS), N, valid(kN));
+      nf = face64<1, ORDER, ALLV, TY>(s, C, kC, N, kN, syC, syN);
+      Nh = N.h;
+    }
+    __syncwarp();  // this warp's xe and sxw
+    double *hout = (double *)in.h[1 - cur];
+    double *qxout = (double *)in.qx[1 - cur];
+    double *qyout = (double *)in.qy[1 - cur];
+    double *hmaxg = (double *)in.h_max;
+    const bool infil = SOURCES && in.cum != nullptr;
+    const bool stations = SOURCES && in.rain_station != nullptr;
+    const bool fwd_tile = (y0 < HB_PAD_Y && in.halo_up[0] != nullptr) ||
+                          (y0 + TY > in.rows - HB_PAD_Y && in.halo_down[0] != nullptr);
+    const int rx = x0 + j;
+#pragma unroll 1
+    for (int i = r0; i < r0 + R; ++i) {
+      const int ry = y0 + i;
+      const size_t go = (size_t)(ry + HB_PAD_Y) * P + (rx + HB_PAD_X);
+      unsigned sid = 0;
+      double F0 = 0.0;
+      if constexpr (SOURCES) {  // loaded ahead of the faces
+        if (stations) sid = __ldg(in.rain_station + go);
+        if (infil) F0 = ((const double *)in.cum)[go];
+      }
+      // --- west face; its flux is the west lane's east face
+      double ehf, exf, eyf, eaf;
+      double dh, dx_, dy_;   // flux differences (minus-side faces - plus-side faces)
+      double wfh, Wh, Eh;
+      bool vW, vE;
+      {
+        const Cel64 W = V.cell(i, j - 1), E = V.cell(i, j + 1);
+        const uint8_t kW = V.code(i, j - 1), kE = V.code(i, j + 1);
+        vW = valid(kW);
+        vE = valid(kE);
+        Wh = W.h;
+        Eh = E.h;
+        const Cel64 sxC = slope64<ORDER, ALLV>(C, W, vW, E, vE);
+        Cel64 sxW{0.0, 0.0, 0.0, 0.0};
+        sxW.z = __shfl_up_sync(0xffffffffu, sxC.z, 1);
+        if constexpr (ORDER == 2) {
+          sxW.h = __shfl_up_sync(0xffffffffu, sxC.h, 1);
+          sxW.qx = __shfl_up_sync(0xffffffffu, sxC.qx, 1);
+          sxW.qy = __shfl_up_sync(0xffffffffu, sxC.qy, 1);
+        }
+        if (lane == 0) sxW = Cel64{s.sxw[i][0], s.sxw[i][1], s.sxw[i][2], s.sxw[i][3]};
+        const Fc64 wf = face64<0, ORDER, ALLV, TY>(s, W, kW, C, kC, sxW, sxC);
+        ehf = __shfl_down_sync(0xffffffffu, wf.fh, 1);
+        exf = __shfl_down_sync(0xffffffffu, wf.fx, 1);
+        eyf = __shfl_down_sync(0xffffffffu, wf.fy, 1);
+        eaf = __shfl_down_sync(0xffffffffu, wf.sa, 1);
+        if (lane == 31) {
+          ehf = s.xe[i][0];
+          exf = s.xe[i][1];
+          eyf = s.xe[i][2];
+          eaf = s.xe[i][3];
+        }
+        dh = sb(wf.fh, ehf);
+        dx_ = ad(sb(sb(wf.fx, exf), eaf), wf.sb);
+        dy_ = sb(wf.fy, eyf);
+        wfh = wf.fh;
+      }
+      // --- south face: the next row's north face
+      const Cel64 SS = V.cell(i + 2, j);
+      const uint8_t kSS = V.code(i + 2, j);
+      const Cel64 syS = slope64<ORDER, ALLV>(Sx, SS, valid(kSS), C, valid(kC));
+      const Fc64 sf = face64<1, ORDER, ALLV, TY>(s, Sx, kS, C, kC, syS, syC);
+
+      // --- cell update
+      if (valid(kC)) {
+        bool active = first || C.h > hs;
+        if (!active) {
+          if constexpr (ALLV) {
+            active = Eh > hs || Nh > hs || Wh > hs || Sx.h > hs;
+          } else {
+            auto nb = [&](bool v, int yy, int xx, double hh) {
+              return v && !(yy == bug_y && xx == bug_x) && hh > hs;
+            };
+            active = nb(vE, ry, rx + 1, Eh) || nb(valid(kN), ry - 1, rx, Nh) ||
+                     nb(vW, ry, rx - 1, Wh) || nb(valid(kS), ry + 1, rx, Sx.h);
+          }
+        }
+        double hu = mu(ad(dh, sb(sf.fh, nf.fh)), r);
+        double qxu = mu(ad(dx_, sb(sf.fx, nf.fx)), r);
+        double qyu = mu(ad(dy_, ad(sb(sb(sf.fy, nf.fy), nf.sa), sf.sb)), r);
+        if (!active) hu = qxu = qyu = 0.0;
+        if constexpr (!ALLV) {
+          // outflow through boundary faces of active cells
+          const bool bE = !vE, bW = !vW, bN = !valid(kN), bS = !valid(kS);
+          if (active && (bE | bW | bN | bS)) {
+            double o = 0.0;
+            if (bE) o += ehf;
+            if (bN) o += nf.fh;
+            if (bW) o -= wfh;
+            if (bS) o -= sf.fh;
+            outf += o;
+          }
+        }
+        // rain (HP/SWE_CUDA.py:549 / HC/stationPrecipitation_Kernel.cu:27)
+        if (stations) hu = ad(hu, mu(__ldcg(in.station_rate + sid), dt));
+        else hu = ad(hu, rdt);
+        if (infil && active) {
+          // Green-Ampt infiltration on the active cells, after rain
+          // (HC/infiltrationCUDA_Kernel.cu:20-46; order HP/CatchFlood_main.py:164-170)
+          const int zc = kC & 15;
+          const double K = in.ks[zc];
+          const double a = ad(F0, mu(dt, K));
+          const double F1 =
+              mu(0.5, ad(a, sqrt(fm(a, a, mu(mu(mu(mu(4.0, dt), K), ad(in.psi[zc], C.h)),
+                                            in.dtheta[zc])))));
+          const double dF = min64(C.h, sb(F1, F0));
+          ((double *)in.cum)[go] = ad(F0, dF);
+          hu = sb(hu, dF);
+        }
+        // implicit friction + update (HC/friction_implicit_andUpdate_jh_Kernel.cu:22-146):
+        // temp = q (sqrt(1 + 4 a |q|) - 1) / (2 a |q|), a = dt C_f / h^2, in the
+        // reference's form of the root's difference (its rounding included)
+        const double h = ad(C.h, hu);
+        double qx = 0.0, qy = 0.0;
+        const bool wet = !(h < hs);
+        if (wet) {
+          qx = ad(C.qx, qxu);
+          qy = ad(C.qy, qyu);
+          const double ih = rcp64(h);
+          const double n = s.manning[kC & 15];
+          if (n > 0.0) {
+            const double qn = sqrt64(fm(qx, qx, mu(qy, qy)));
+            const double a = mu(mu(mu(mu(mu(dt, g), mu(n, n)), rcbrt(h)), ih), ih);
+            const double x = mu(a, qn);
+            const double S = __dsqrt_rn(fm(4.0, x, 1.0));
+            const double f = mu(sb(S, 1.0), rcp64(mu(2.0, x)));
+            const double lim2 = mu(mu(mu(25.0 * kG, h), h), h);  // (5 h sqrt(g h))^2
+            auto limit = [&](double q) {
+              const double temp = mu(q, f);
+              const double q2 = fm(2.0, temp, -q);
+              const double over = (__double2hiint(q2) ^ __double2hiint(temp)) < 0 ? 0.0 : q2;
+              const double t = mu(temp, temp) > lim2 ? over : temp;
+              return fabs(q) > 1.0e-10 ? t : q;
+            };
+            qx = limit(qx);
+            qy = limit(qy);
+          }
+          if (h > hs) {
+            // CFL speed (HC/timeControl_Kernel.cu:186-189), its root in single precision
+            const double sp = fm(max64(fabs(qx), fabs(qy)), ih,
+                                 (double)__fsqrt_rn((float)mu(g, h)));
+            smax = max64(smax, sp);
+          }
+        }
+        if (!(h > hs)) any_dry = 1;
+        hout[go] = h;
+        qxout[go] = qx;
+        qyout[go] = qy;
+        const double hm = s.hmax[i * kTW + j];
+        hmaxg[go] = h > hm ? h : hm;
+        if (fwd_tile) {
+          // into the neighbour strip's halo row of the same output buffer (plain
+          // stores; the neighbour's arrays may be on a peer GPU)
+          const int ob = 1 - cur;
+          auto fwd = [&](void *const *dst, int row) {
+            const size_t gh = (size_t)row * P + (rx + HB_PAD_X);
+            ((double *)dst[ob])[gh] = h;
+            ((double *)dst[2 + ob])[gh] = qx;
+            ((double *)dst[4 + ob])[gh] = qy;
+          };
+          if (ry < HB_PAD_Y && in.halo_up[0] != nullptr)
+            fwd(in.halo_up, in.halo_up_rows + HB_PAD_Y + ry);
+          if (ry >= in.rows - HB_PAD_Y && in.halo_down[0] != nullptr)
+            fwd(in.halo_down, ry - in.rows + HB_PAD_Y);
+          // system-wide order before this block's partial, its count and the
+          // host's next collective
+          __threadfence_system();
+        }
+        vol = ad(vol, h);
+      }
+      // slide the column window down one row
+      nf = sf;
+      Nh = C.h;
+      kN = kC;
+      C = Sx;
+      kC = kS;
+      Sx = SS;
+      kS = kSS;
+      syC = syS;
+    }
+  }
+
+  // --- partials and the instance's last-tile finalize
+  vol = warp_sum(vol);
+  if constexpr (!ALLV) outf = warp_sum(outf);
+  smax = warp_max(smax);
+  any_dry = __any_sync(0xffffffffu, any_dry);
+  if (lane == 0) {
+    s.red_d[0][w] = vol;
+    s.red_d[1][w] = outf;
+    s.red_s[w] = smax;
+    s.red_i[w] = any_dry;
+  }
+  __syncthreads();
+  const int n_inst_tiles = in.tiles_x * in.tiles_y * kPer;
+  const int gt = group_tiles(n_inst_tiles);
+  const int grp = lt / gt;
+  const int gsize = min(gt, n_inst_tiles - grp * gt);
+  const int gbase = tile0 / kGroupTiles + ii;
+  if (tid == 0) {
+    partials[tile] = block_sum<kRowsNT>(s.red_d, s.red_s, s.red_i);
+    cuda::atomic_ref<unsigned, cuda::thread_scope_device> done(gcount[gbase + grp]);
+    s.last = (done.fetch_add(1u, cuda::memory_order_acq_rel) == (unsigned)(gsize - 1));
+  }
+  __syncthreads();
+  if (s.last)
+    close_group<double, kRowsNT>(in, ii, partials + tile0 + grp * gt, gsize, gparts, gcount,
+                                 gbase + grp, gbase, (n_inst_tiles + gt - 1) / gt, bct, s.red_d,
+                                 s.red_s, s.red_i, &s.last2);
+  __syncthreads();
+  return true;
+}
+
+// The general path out of line, so that the all-valid path keeps its own
+// register allocation.
+template <int TY, bool SOURCES, int ORDER>
+__device__ __noinline__ bool rows64_general(Rows64Smem<TY> &s, unsigned &phase, const TileEntry en,
+                                            const hb_instance *__restrict__ insts,
+                                            TilePartial *__restrict__ partials,
+                                            TilePartial *__restrict__ gparts,
+                                            unsigned *__restrict__ gcount,
+                                            BcTable *__restrict__ bct,
+                                            const CUtensorMap *__restrict__ maps) {
+  return rows64_tile<TY, SOURCES, false, ORDER>(s, phase, en, insts, partials, gparts, gcount,
+                                                bct, maps);
+}
+
+// The FP64 step: one programmatic launch over the prepared list (general
+// blocks with a valid cell [0, n_live), all-valid blocks [n_live,
+// n_valid_end), blocks without a valid cell), one CTA per block or a smaller
+// grid that loops.  `order` (whole tiles only) stands in for the list.
+template <int TY, bool SOURCES, int ORDER>
+__global__ void __launch_bounds__(kRowsNT, 4)
+rows64_kernel(const hb_instance *__restrict__ insts, const TileEntry *__restrict__ list,
+              const int n_live, const int n_valid_end, const int n_list,
+              TilePartial *__restrict__ partials, TilePartial *__restrict__ gparts,
+              unsigned *__restrict__ gcount, BcTable *__restrict__ bct,
+              const CUtensorMap *__restrict__ maps, const int32_t *__restrict__ order,
+              const int32_t *__restrict__ tile_inst) {
+  using S = Rows64Smem<TY>;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  S &s = *reinterpret_cast<S *>(smem_raw);
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (threadIdx.x == 0) {
+    mbar_init(&s.bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  unsigned phase = 0;
+  for (int k = blockIdx.x; k < n_list; k += gridDim.x) {
+    TileEntry en;
+    if (TY == 32 && order) {
+      en.tile = order[k];
+      en.inst = tile_inst[en.tile < 0 ? ~en.tile : en.tile];
+      en.ctrl = insts[en.inst].ctrl;
+    } else {
+      en = list[k];
+    }
+    const bool ok = k >= n_live && k < n_valid_end
+                        ? rows64_tile<TY, SOURCES, true, ORDER>(s, phase, en, insts, partials,
+                                                                gparts, gcount, bct, maps)
+                        : rows64_general<TY, SOURCES, ORDER>(s, phase, en, insts, partials,
+                                                             gparts, gcount, bct, maps);
+    if (!ok) return;
+  }
+}
