@@ -1134,17 +1134,19 @@ pairs_mixed_kernel(const hb_instance *__restrict__ insts, const TileEntry *__res
   using S = PairSmem<TY>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   S &s = *reinterpret_cast<S *>(smem_raw);
-  // Programmatic launch: the next kernel's CTAs may take their slots once every
-  // CTA of this grid has started, and this one waits here for the kernel before
-  // it; everything that kernel may have written is read after the wait.  Hides
-  // the launch gap: 90.1 -> 87.7 us a step on 2048^2, 27.2 -> 25.7 on 256^2.
-  asm volatile("griddepcontrol.launch_dependents;");
+  // Programmatic launch: this kernel waits here for the one before it (whatever
+  // that may have written is read after the wait) and then lets the next
+  // kernel's CTAs take free slots, once every CTA of this grid has started.
+  // Hides the launch gap: 90.1 -> 87.7 us a step on 2048^2, 27.2 -> 25.7 on
+  // 256^2.  (Released before the wait, several kernels of a small grid queue up
+  // on the SMs and crowd each other's placement: 256^2 14.2 -> 17.1 us.)
   if (threadIdx.x == 0) {
     mbar_init(&s.bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
   unsigned phase = 0;
   if constexpr (TY != 32) {
     for (int k = blockIdx.x; k < n_list; k += gridDim.x) {

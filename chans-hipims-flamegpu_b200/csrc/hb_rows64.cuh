@@ -578,6 +578,9 @@ __device__ __forceinline__ bool rows64_tile(Rows64Smem<TY> &s, unsigned &phase, 
     }
   }
 
+  // the next step's CTAs may take this one's slots from here on (from the start
+  // of the block instead: 512^2 26.2 -> 28.8 us a step, 301 x 517 20.4 -> 22.4)
+  if constexpr (TY != 32) asm volatile("griddepcontrol.launch_dependents;");
   // --- partials and the instance's last-tile finalize
   vol = warp_sum(vol);
   if constexpr (!ALLV) outf = warp_sum(outf);
@@ -638,13 +641,13 @@ rows64_kernel(const hb_instance *__restrict__ insts, const TileEntry *__restrict
   using S = Rows64Smem<TY>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   S &s = *reinterpret_cast<S *>(smem_raw);
-  asm volatile("griddepcontrol.launch_dependents;");
   if (threadIdx.x == 0) {
     mbar_init(&s.bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if constexpr (TY == 32) asm volatile("griddepcontrol.launch_dependents;");
   unsigned phase = 0;
   for (int k = blockIdx.x; k < n_list; k += gridDim.x) {
     TileEntry en;
