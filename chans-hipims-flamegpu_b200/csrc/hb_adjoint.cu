@@ -5,9 +5,9 @@
 // (dU^{n+1}/dtheta)^T lambda^{n+1} for theta = (Manning n of each zone, rain
 // multiplier), with the time step frozen (the forward's dt schedule replayed).
 // Two passes per step over the dense raster of one catchment:
-//  1. cells: recompute the cell's four faces and its update, reverse the
-//     update (friction, rain), write the direct part of lambda^n and mu =
-//     dJ/d(flux increments) of active cells;
+//  1. cells: recompute the block's faces (once each, in shared memory) and the
+//     cell's update, reverse the update (friction, rain), write the direct part
+//     of lambda^n and mu = dJ/d(flux increments) of active cells;
 //  2. faces: every face once, owned by its east / south cell; reverse it with
 //     the adjoints of its two cells' increments and scatter the result to its
 //     four input cells with FP64 atomics.
@@ -37,15 +37,16 @@ struct Grid {
     return (size_t)(r + HB_PAD_Y) * P + (c + HB_PAD_X);
   }
   __device__ __forceinline__ uint8_t cd(int r, int c) const {
-    if (r < 0 || c < 0 || r >= rows || c >= cols) return (uint8_t)(HB_NODATA_CLASS << 4);
+    if ((unsigned)r >= (unsigned)rows || (unsigned)c >= (unsigned)cols)
+      return (uint8_t)(HB_NODATA_CLASS << 4);
     return code[(size_t)(r + HB_PAD_Y) * CP + (c + HB_CODE_PAD_X)];
   }
   __device__ __forceinline__ bool valid(int r, int c) const {
     return (cd(r, c) >> 4) != HB_NODATA_CLASS;
   }
+  // (r, c) within two cells of the raster: the dense arrays hold that margin
   __device__ __forceinline__ Cz cell(int r, int c) const {
-    Cz v{0, 0, 0, 0};
-    if (r < -HB_PAD_Y || c < -HB_PAD_X || r >= rows + 2 || c >= cols + 2) return v;
+    Cz v;
     const size_t k = off(r, c);
     v.h = h[k];
     v.qx = qx[k];
@@ -156,53 +157,61 @@ __device__ FaceOut5 face_at(const Grid &G, const BcVals &bc, int ra, int ca, int
   return o;
 }
 
-// Face values kept by the optional face pass: x-face (r, c-1)|(r, c) and
-// y-face (r, c)|(r-1, c) of index r * (cols + 1) + c, fields fh, fx, fy, sa, sb.
-__device__ __forceinline__ FaceOut5 load_face(const hb_adjoint_args &a, int dir, int r, int c) {
-  const double *f = a.faces + (size_t)dir * 5 * a.face_stride + (size_t)r * (a.cols + 1) + c;
-  const int64_t s = a.face_stride;
-  return FaceOut5{f[0], f[s], f[2 * s], f[3 * s], f[4 * s]};
+// Whether the face between (ra, ca) and (rb, cb) needs the boundary tables
+// (exactly one valid side).
+__device__ __forceinline__ bool is_ghost_face(const Grid &G, int ra, int ca, int rb, int cb) {
+  return G.valid(ra, ca) != G.valid(rb, cb);
 }
 
-// Pass 0 (optional): every face once, forward only, into a.faces.
-__global__ void __launch_bounds__(128)
-adj_facefwd_kernel(hb_adjoint_args a) {
-  __shared__ BcVals bc;
-  const hb_instance &in = *a.instance;
-  Grid G{a.instance, a.rows, a.cols, a.pitch, a.code_pitch, a.h, a.qx, a.qy,
-         (const double *)in.z, in.code};
-  load_bc(in, a.t, bc);
-  __syncthreads();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y * blockDim.y + threadIdx.y;
-  if (r > a.rows || c > a.cols) return;
-  const size_t idx = (size_t)r * (a.cols + 1) + c;
-  const int64_t s = a.face_stride;
-  FaceOut5 x{0, 0, 0, 0, 0}, y{0, 0, 0, 0, 0};
-  if (r < a.rows) x = face_at<0>(G, bc, r, c - 1, r, c, nullptr, nullptr, nullptr, nullptr);
-  if (c < a.cols) y = face_at<1>(G, bc, r, c, r - 1, c, nullptr, nullptr, nullptr, nullptr);
-  double *fx = a.faces + idx, *fy = a.faces + 5 * s + idx;
-  fx[0] = x.fh; fx[s] = x.fx; fx[2 * s] = x.fy; fx[3 * s] = x.sa; fx[4 * s] = x.sb;
-  fy[0] = y.fh; fy[s] = y.fx; fy[2 * s] = y.fy; fy[3 * s] = y.sa; fy[4 * s] = y.sb;
-}
-
-// Pass 1: per cell.
-__global__ void __launch_bounds__(256)
+// Pass 1: a block of 32 x 8 cells and nine warps.  Each face of the block's
+// cells is evaluated once into shared memory (warps 0-7: the west and north
+// faces of their row's cells; warp 8: the last row of y-faces and the last
+// column of x-faces), then the cells are updated and reversed.  FP64 issue and
+// latency bind it (45 % of issue slots).  With the faces in a pass of their own
+// through global memory, IEEE divisions, pow and the boundary tables searched by
+// every block, the two passes took 27 + 41 us (512^2 cells, cold); 34 us so.
+constexpr int kCellRows = 8;
+__global__ void __launch_bounds__(32 * (kCellRows + 1), 2)
 adj_cell_kernel(hb_adjoint_args a) {
   __shared__ BcVals bc;
-  __shared__ double red[HB_MAX_ZONES + 1][8];
+  __shared__ double red[HB_MAX_ZONES + 1][kCellRows + 1];
+  __shared__ double sx[5][kCellRows][33], sy[5][kCellRows + 1][32];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const hb_instance &in = *a.instance;
   Grid G{a.instance, a.rows, a.cols, a.pitch, a.code_pitch, a.h, a.qx, a.qy,
          (const double *)in.z, in.code};
-  load_bc(in, a.t, bc);
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  if (tid < (HB_MAX_ZONES + 1) * 8) (&red[0][0])[tid] = 0.0;
+  const int lane = threadIdx.x, w = threadIdx.y;
+  const int tid = lane + 32 * w;
+  for (int q = tid; q < (HB_MAX_ZONES + 1) * (kCellRows + 1); q += 32 * (kCellRows + 1))
+    (&red[0][0])[q] = 0.0;
+  const int r0 = blockIdx.y * kCellRows, c0 = blockIdx.x * 32;
+  const int r = r0 + w, c = c0 + lane;
+  // this thread's x-face (rx, cx - 1) | (rx, cx) and y-face (r, c) | (r - 1, c)
+  const bool extra = w == kCellRows;  // the last warp's x-faces: column c0 + 32, row = lane
+  const int rx = extra ? r0 + lane : r, cx = extra ? c0 + 32 : c;
+  const bool hasx = (!extra || lane < kCellRows) && rx < a.rows && cx <= a.cols;
+  const bool hasy = r <= a.rows && c < a.cols;
+  const bool ghosts = (hasx && is_ghost_face(G, rx, cx - 1, rx, cx)) ||
+                      (hasy && is_ghost_face(G, r, c, r - 1, c));
+  if (__syncthreads_or(ghosts)) {  // boundary tables: blocks with ghost faces only
+    load_bc(in, a.t, bc);
+    __syncthreads();
+  }
+  if (hasx) {
+    const FaceOut5 f = face_at<0>(G, bc, rx, cx - 1, rx, cx, nullptr, nullptr, nullptr, nullptr);
+    const int i = rx - r0, j = cx - c0;
+    sx[0][i][j] = f.fh; sx[1][i][j] = f.fx; sx[2][i][j] = f.fy; sx[3][i][j] = f.sa;
+    sx[4][i][j] = f.sb;
+  }
+  if (hasy) {
+    const FaceOut5 f = face_at<1>(G, bc, r, c, r - 1, c, nullptr, nullptr, nullptr, nullptr);
+    sy[0][w][lane] = f.fh; sy[1][w][lane] = f.fx; sy[2][w][lane] = f.fy; sy[3][w][lane] = f.sa;
+    sy[4][w][lane] = f.sb;
+  }
   __syncthreads();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y * blockDim.y + threadIdx.y;
   double gz = 0.0, gm = 0.0;
   int zone = 0;
-  if (r < a.rows && c < a.cols) {
+  if (!extra && r < a.rows && c < a.cols) {
     const size_t k = G.off(r, c);
     double *mu_h = a.mu, *mu_qx = a.mu + a.mu_stride, *mu_qy = a.mu + 2 * a.mu_stride;
     if (!G.valid(r, c)) {
@@ -210,6 +219,7 @@ adj_cell_kernel(hb_adjoint_args a) {
       mu_h[k] = mu_qx[k] = mu_qy[k] = 0.0;
     } else {
       const Cz u = G.cell(r, c);
+      const C3 ob{a.lam_h[k], a.lam_qx[k], a.lam_qy[k]};
       const double hs = kHs;
       // fluxMask activity (HC/fluxMaskGenerator_Kernel.cu:19-42, cell 0 ignored)
       bool active = a.first || u.h > hs;
@@ -221,21 +231,12 @@ adj_cell_kernel(hb_adjoint_args a) {
       const double kk = a.dt / in.dx;
       C3 rr{0, 0, 0};
       if (active) {
-        FaceOut5 fe, fw, fn, fs;
-        if (a.faces) {
-          fe = load_face(a, 0, r, c + 1);
-          fw = load_face(a, 0, r, c);
-          fn = load_face(a, 1, r, c);
-          fs = load_face(a, 1, r + 1, c);
-        } else {
-          fe = face_at<0>(G, bc, r, c, r, c + 1, nullptr, nullptr, nullptr, nullptr);
-          fw = face_at<0>(G, bc, r, c - 1, r, c, nullptr, nullptr, nullptr, nullptr);
-          fn = face_at<1>(G, bc, r, c, r - 1, c, nullptr, nullptr, nullptr, nullptr);
-          fs = face_at<1>(G, bc, r + 1, c, r, c, nullptr, nullptr, nullptr, nullptr);
-        }
-        rr.h = ((fw.fh + fs.fh) - (fe.fh + fn.fh)) * kk;
-        rr.qx = ((fw.fx + fs.fx) - (fe.fx + fn.fx) - fe.sa + fw.sb) * kk;
-        rr.qy = ((fw.fy + fs.fy) - (fe.fy + fn.fy) - fn.sa + fs.sb) * kk;
+        const int j = lane;
+        rr.h = ((sx[0][w][j] + sy[0][w + 1][j]) - (sx[0][w][j + 1] + sy[0][w][j])) * kk;
+        rr.qx = ((sx[1][w][j] + sy[1][w + 1][j]) - (sx[1][w][j + 1] + sy[1][w][j]) -
+                 sx[3][w][j + 1] + sx[4][w][j]) * kk;
+        rr.qy = ((sx[2][w][j] + sy[2][w + 1][j]) - (sx[2][w][j + 1] + sy[2][w][j]) -
+                 sy[3][w][j] + sy[4][w + 1][j]) * kk;
       }
       rr.h += a.rain_rate * a.dt;
       zone = G.cd(r, c) & 15;
@@ -243,7 +244,6 @@ adj_cell_kernel(hb_adjoint_args a) {
       CellTape tp;
       const C3 uu{u.h, u.qx, u.qy};
       cell_fwd(uu, rr, n, a.dt, tp);
-      const C3 ob{a.lam_h[k], a.lam_qx[k], a.lam_qy[k]};
       C3 ub, rb;
       double nb;
       cell_rev(tp, ob, a.dt, ub, rb, nb);
@@ -263,61 +263,74 @@ adj_cell_kernel(hb_adjoint_args a) {
       gm = rb.h * a.rain_base * a.dt;
     }
   }
-  // block reduction of the parameter gradient (zones are few)
-  const int lane = tid & 31, wid = tid >> 5;
-  for (int zz = 0; zz < HB_MAX_ZONES; zz++) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  // block reduction of the parameter gradient: each warp sums the zones it
+  // holds (one or two as a rule)
+  for (unsigned rem = __ballot_sync(0xffffffffu, gz != 0.0); rem;) {
+    const int zz = __shfl_sync(0xffffffffu, zone, __ffs(rem) - 1);
     double v = (zone == zz) ? gz : 0.0;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[zz][wid] = v;
+    if (lane == 0) red[zz][w] = v;
+    rem &= ~__ballot_sync(0xffffffffu, zone == zz);
   }
   for (int o = 16; o > 0; o >>= 1) gm += __shfl_xor_sync(0xffffffffu, gm, o);
-  if (lane == 0) red[HB_MAX_ZONES][wid] = gm;
+  if (lane == 0) red[HB_MAX_ZONES][w] = gm;
   __syncthreads();
   if (tid <= HB_MAX_ZONES) {
     double v = 0;
-    for (int w = 0; w < (int)(blockDim.x * blockDim.y) / 32; w++) v += red[tid][w];
+    for (int q = 0; q < kCellRows; q++) v += red[tid][q];
     if (v != 0.0) atomicAdd(a.grad + tid, v);
   }
 }
 
-// Pass 2: per face, owned by its east (x) / south (y) cell.
-__global__ void __launch_bounds__(128)
-adj_face_kernel(hb_adjoint_args a) {
-  __shared__ BcVals bc;
-  const hb_instance &in = *a.instance;
-  Grid G{a.instance, a.rows, a.cols, a.pitch, a.code_pitch, a.h, a.qx, a.qy,
-         (const double *)in.z, in.code};
-  load_bc(in, a.t, bc);
-  __syncthreads();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = blockIdx.y * blockDim.y + threadIdx.y;
-  if (r > a.rows || c > a.cols) return;
-  const double kk = a.dt / in.dx;
+// Pass 2: every face along DIR (x: owned by its east cell, y: by its south
+// cell); blockIdx.z selects the direction, which halves a thread's chain and
+// evens out the last wave.  Bound by latency at 16 warps an SM (the decision
+// tape of a face fills 128 registers; 156 without the cap, 3 % slower): 62 us a
+// step of 512^2 cells with both directions in one thread and IEEE divisions,
+// 37 us so (cold).
+template <int DIR>
+__device__ __forceinline__ void face_rev_at(const hb_adjoint_args &a, const Grid &G,
+                                            const hb_instance &in, BcVals &bc, int r, int c) {
+  const int ra = r, ca = DIR == 0 ? c - 1 : c, rb = DIR == 0 ? r : r - 1, cb = c;
   const double *mu_h = a.mu, *mu_qx = a.mu + a.mu_stride, *mu_qy = a.mu + 2 * a.mu_stride;
-  auto mu = [&](int rr, int cc) {
+  const bool has = DIR == 0 ? (r < a.rows && c <= a.cols) : (r <= a.rows && c < a.cols);
+  const bool va = has && G.valid(ra, ca), vb = has && G.valid(rb, cb);
+  auto mu = [&](bool v, int rr, int cc) {
     C3 m{0, 0, 0};
-    if (rr >= 0 && cc >= 0 && rr < a.rows && cc < a.cols && G.valid(rr, cc)) {
+    if (v) {
       const size_t k = G.off(rr, cc);
       m = C3{mu_h[k], mu_qx[k], mu_qy[k]};
     }
     return m;
   };
-  // x-face between (r, c-1) = A and (r, c) = B
-  if (r < a.rows) {
-    const C3 mA = mu(r, c - 1), mB = mu(r, c);
-    const FaceOut5 ob{kk * (mB.h - mA.h), kk * (mB.qx - mA.qx), kk * (mB.qy - mA.qy),
-                      -kk * mA.qx, kk * mB.qx};
-    if (ob.fh != 0.0 || ob.fx != 0.0 || ob.fy != 0.0 || ob.sa != 0.0 || ob.sb != 0.0)
-      face_at<0>(G, bc, r, c - 1, r, c, &ob, a.out_h, a.out_qx, a.out_qy, a.h_reg);
+  const double kk = a.dt / in.dx;
+  const C3 mA = mu(va, ra, ca), mB = mu(vb, rb, cb);
+  const FaceOut5 ob{kk * (mB.h - mA.h), kk * (mB.qx - mA.qx), kk * (mB.qy - mA.qy),
+                    -kk * (DIR == 0 ? mA.qx : mA.qy), kk * (DIR == 0 ? mB.qx : mB.qy)};
+  const bool work = (va || vb) && (ob.fh != 0.0 || ob.fx != 0.0 || ob.fy != 0.0 ||
+                                   ob.sa != 0.0 || ob.sb != 0.0);
+  if (__syncthreads_or(work && va != vb)) {  // boundary tables: blocks with ghost faces only
+    load_bc(in, a.t, bc);
+    __syncthreads();
   }
-  // y-face between (r, c) = A (south) and (r - 1, c) = B (north)
-  if (c < a.cols) {
-    const C3 mA = mu(r, c), mB = mu(r - 1, c);
-    const FaceOut5 ob{kk * (mB.h - mA.h), kk * (mB.qx - mA.qx), kk * (mB.qy - mA.qy),
-                      -kk * mA.qy, kk * mB.qy};
-    if (ob.fh != 0.0 || ob.fx != 0.0 || ob.fy != 0.0 || ob.sa != 0.0 || ob.sb != 0.0)
-      face_at<1>(G, bc, r, c, r - 1, c, &ob, a.out_h, a.out_qx, a.out_qy, a.h_reg);
-  }
+  if (work) face_at<DIR>(G, bc, ra, ca, rb, cb, &ob, a.out_h, a.out_qx, a.out_qy, a.h_reg);
+}
+
+__global__ void __launch_bounds__(128, 4)
+adj_face_kernel(hb_adjoint_args a) {
+  __shared__ BcVals bc;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const hb_instance &in = *a.instance;
+  Grid G{a.instance, a.rows, a.cols, a.pitch, a.code_pitch, a.h, a.qx, a.qy,
+         (const double *)in.z, in.code};
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = blockIdx.y * blockDim.y + threadIdx.y;
+  if (blockIdx.z == 0)
+    face_rev_at<0>(a, G, in, bc, r, c);
+  else
+    face_rev_at<1>(a, G, in, bc, r, c);
+  asm volatile("griddepcontrol.launch_dependents;");
 }
 
 __global__ void gauge_kernel(int64_t n, const int64_t *off, const double *h, const double *obs,
@@ -340,24 +353,24 @@ extern "C" int hb_adjoint_step(const hb_adjoint_args *a, void *stream) {
   if (a->faces && a->face_stride < (int64_t)(a->rows + 1) * (a->cols + 1))
     return set_error(HB_ERR_ARG, "hb_adjoint_step: face_stride below (rows + 1) * (cols + 1)");
   auto st = as_stream(stream);
-  if (a->faces) {
-    const dim3 blk0(32, 4);
-    const dim3 g0((a->cols + 1 + 31) / 32, (a->rows + 1 + 3) / 4);
-    adj_facefwd_kernel<<<g0, blk0, 0, st>>>(*a);
-    int rc0 = check_launch("hb_adjoint_step (faces forward)");
-    if (rc0) return rc0;
+  // Programmatic launches: each kernel waits for the one before it at its top.
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cfg.blockDim = dim3(32, kCellRows + 1);
+  cfg.gridDim = dim3((a->cols + 31) / 32, (a->rows + kCellRows - 1) / kCellRows);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, adj_cell_kernel, *a);
+  if (e == cudaSuccess) {
+    cfg.blockDim = dim3(32, 4);
+    cfg.gridDim = dim3((a->cols + 1 + 31) / 32, (a->rows + 1 + 3) / 4, 2);
+    e = cudaLaunchKernelEx(&cfg, adj_face_kernel, *a);
   }
-  const dim3 blk(32, 8);
-  const dim3 g1((a->cols + 31) / 32, (a->rows + 7) / 8);
-  adj_cell_kernel<<<g1, blk, 0, st>>>(*a);
-  int rc = check_launch("hb_adjoint_step (cells)");
-  if (rc) return rc;
-  // 128-thread blocks: the face pass needs ~156 registers a thread, so three
-  // blocks (12 warps) fit an SM where one 256-thread block would
-  const dim3 blk2(32, 4);
-  const dim3 g2((a->cols + 1 + 31) / 32, (a->rows + 1 + 3) / 4);
-  adj_face_kernel<<<g2, blk2, 0, st>>>(*a);
-  return check_launch("hb_adjoint_step (faces)");
+  if (e != cudaSuccess) return set_error(HB_ERR_CUDA, "hb_adjoint_step: %s", cudaGetErrorString(e));
+  return check_launch("hb_adjoint_step");
 }
 
 extern "C" int hb_adjoint_gauge(int64_t n, const int64_t *offsets, const double *h,

@@ -1,7 +1,7 @@
 // hb_adjoint.cuh -- reverse-mode derivatives of the HiPIMS step (FP64).
 //
-// The forward functions restate, operation for operation, the FP64 path of
-// the fused step (hb_fused.cu, itself following the reference kernels
+// The forward functions restate the FP64 step (hb_rows64.cuh, itself following
+// the reference kernels
 // HC/flucCal_2ndOrder_jh_improved_Kernel.cu:43-506 and
 // HC/friction_implicit_andUpdate_jh_Kernel.cu:22-146); the reverse functions
 // propagate adjoints back through them with every discrete decision (minmod
@@ -9,8 +9,14 @@
 // friction limiter) taken as the forward takes it.  The functions are
 // __host__ __device__ so that tests can check them against finite
 // differences on the CPU.
+//
+// On the device, reciprocals and roots are those of hb_fp64.cuh (an IEEE
+// division is some twenty-five instructions, and a reverse face had fifteen);
+// on the host they are the plain operations.
 #pragma once
 #include <math.h>
+
+#include "hb_fp64.cuh"
 
 #ifdef __CUDACC__
 #define HB_HD __host__ __device__ __forceinline__
@@ -23,6 +29,28 @@ namespace adj {
 
 constexpr double kHs = 1.0e-6;
 constexpr double kG = 9.81;
+
+HB_HD double rcp(double x) {
+#ifdef __CUDA_ARCH__
+  return rcp64(x);
+#else
+  return 1.0 / x;
+#endif
+}
+HB_HD double root(double x) {
+#ifdef __CUDA_ARCH__
+  return sqrt64(x);
+#else
+  return sqrt(x);
+#endif
+}
+HB_HD double inv_cbrt(double x) {
+#ifdef __CUDA_ARCH__
+  return rcbrt(x);
+#else
+  return 1.0 / cbrt(x);
+#endif
+}
 
 struct C3 {  // a cell's prognostic state or its adjoint
   double h, qx, qy;
@@ -85,6 +113,7 @@ struct FaceTape {
   bool wetA, wetB;
   double eLh, eLz, eLqx, eLqy, eRh, eRz, eRqx, eRqy;
   bool velL, velR;
+  double il, ir;  // 1 / edge depth, 0 for a dry edge
   double uxl, uyl, uxr, uyr;
   // hydrostatic
   double wlA, wlB, hi, lo;
@@ -140,10 +169,12 @@ HB_HD FaceOut5 face_fwd(const FaceIn &in, FaceTape<DIR> &tp) {
   // velocities before the hydrostatic step
   tp.velL = !(tp.eLh < hs);
   tp.velR = !(tp.eRh < hs);
-  tp.uxl = tp.velL ? tp.eLqx / tp.eLh : 0.0;
-  tp.uyl = tp.velL ? tp.eLqy / tp.eLh : 0.0;
-  tp.uxr = tp.velR ? tp.eRqx / tp.eRh : 0.0;
-  tp.uyr = tp.velR ? tp.eRqy / tp.eRh : 0.0;
+  tp.il = tp.velL ? rcp(tp.eLh) : 0.0;
+  tp.ir = tp.velR ? rcp(tp.eRh) : 0.0;
+  tp.uxl = tp.eLqx * tp.il;
+  tp.uyl = tp.eLqy * tp.il;
+  tp.uxr = tp.eRqx * tp.ir;
+  tp.uyr = tp.eRqy * tp.ir;
   // hydrostatic reconstruction (2nd order)
   tp.wlA = A.z + A.h;
   tp.wlB = B.z + B.h;
@@ -193,11 +224,11 @@ HB_HD FaceOut5 face_fwd(const FaceIn &in, FaceTape<DIR> &tp) {
   if (!tp.bothdry) {
     const double uL = tp.uL, uR = tp.uR, vL = tp.vL, vR = tp.vR;
     const double qxL = uL * hL, qyL = vL * hL, qxR = uR * hR, qyR = vR * hR;
-    tp.aL = sqrt(g * hL);
-    tp.aR = sqrt(g * hR);
+    tp.aL = root(g * hL);
+    tp.aR = root(g * hR);
     tp.base = (tp.aL + tp.aR) / 2.0 + (uL - uR) / 4.0;
     tp.ustar = (uL + uR) / 2.0 + tp.aL - tp.aR;
-    tp.astar = sqrt(g * ((tp.base * tp.base) / g));
+    tp.astar = fabs(tp.base);
     if (hL <= hs) {
       tp.sLcase = 0;
       tp.sL = uR - 2.0 * tp.aR;
@@ -215,19 +246,22 @@ HB_HD FaceOut5 face_fwd(const FaceIn &in, FaceTape<DIR> &tp) {
       tp.sR = b1 >= b2 ? b1 : b2;
     }
     const double sL = tp.sL, sR = tp.sR;
-    const double sM = (sL * hR * (uR - sR) - sR * hL * (uL - sL)) / (hR * (uR - sR) - hL * (uL - sL));
+    // contact speed sM = num / den: its sign
+    const double pL = hL * (uL - sL), pR = hR * (uR - sR);
+    const double num = sL * pR - sR * pL, den = pR - pL;
+    const bool some = den != 0.0, sMpos = some && (num == 0.0 || (num > 0.0) == (den > 0.0));
     tp.hfL = qxL;
     tp.qfL = uL * qxL + 0.5 * g * hL * hL;
     tp.tfL = uL * qyL;
     tp.hfR = qxR;
     tp.qfR = uR * qxR + 0.5 * g * hR * hR;
     tp.tfR = uR * qyR;
-    tp.inv = 1.0 / (sR - sL);
+    tp.inv = rcp(sR - sL);
     tp.hfM = (sR * tp.hfL - sL * tp.hfR + sL * sR * (hR - hL)) * tp.inv;
     tp.qfM = (sR * tp.qfL - sL * tp.qfR + sL * sR * (qxR - qxL)) * tp.inv;
     if (0.0 <= sL) tp.region = 0;
-    else if (sL < 0.0 && 0.0 <= sM) tp.region = 1;
-    else if (sM < 0.0 && 0.0 <= sR) tp.region = 2;
+    else if (sMpos) tp.region = 1;
+    else if (some && 0.0 <= sR) tp.region = 2;
     else tp.region = 3;
     switch (tp.region) {
       case 0: Fh = tp.hfL; Fn = tp.qfL; Ft = tp.tfL; break;
@@ -370,8 +404,8 @@ HB_HD void face_rev(const FaceIn &in, const FaceTape<DIR> &tp, const FaceOut5 &o
     uL_b += 0.25 * base_b;
     uR_b -= 0.25 * base_b;
     // a = sqrt(g h)
-    if (hL > 0.0) Lh_b += aL_b * g / (2.0 * tp.aL);
-    if (hR > 0.0) Rh_b += aR_b * g / (2.0 * tp.aR);
+    if (hL > 0.0) Lh_b += aL_b * (0.5 * g) * rcp(tp.aL);
+    if (hR > 0.0) Rh_b += aR_b * (0.5 * g) * rcp(tp.aR);
     // qxL = uL hL, qyL = vL hL, ...
     uL_b += qxL_b * hL;
     Lh_b += qxL_b * uL + qyL_b * vL;
@@ -435,14 +469,14 @@ HB_HD void face_rev(const FaceIn &in, const FaceTape<DIR> &tp, const FaceOut5 &o
   // velocities: u = q / h (when h >= hs)
   double eLqx_b = 0, eLqy_b = 0, eRqx_b = 0, eRqy_b = 0;
   if (tp.velL) {
-    eLqx_b += uxl_b / tp.eLh;
-    eLqy_b += uyl_b / tp.eLh;
-    eLh_b -= (uxl_b * tp.uxl + uyl_b * tp.uyl) / tp.eLh;
+    eLqx_b += uxl_b * tp.il;
+    eLqy_b += uyl_b * tp.il;
+    eLh_b -= (uxl_b * tp.uxl + uyl_b * tp.uyl) * tp.il;
   }
   if (tp.velR) {
-    eRqx_b += uxr_b / tp.eRh;
-    eRqy_b += uyr_b / tp.eRh;
-    eRh_b -= (uxr_b * tp.uxr + uyr_b * tp.uyr) / tp.eRh;
+    eRqx_b += uxr_b * tp.ir;
+    eRqy_b += uyr_b * tp.ir;
+    eRh_b -= (uxr_b * tp.uxr + uyr_b * tp.uyr) * tp.ir;
   }
   // edges -> cells and slopes (z has no adjoint: the bed is fixed)
   double sA_b[4] = {0, 0, 0, 0}, sB_b[4] = {0, 0, 0, 0};
@@ -523,7 +557,7 @@ HB_HD bool ghost_of(int type, int axis, const Cz &C, double hb, double wlb, doub
 // Cell update after the fluxes: h1 = h + hu; implicit Manning friction on
 // q + qu with the Froude > 5 limiter (reference form and decisions).
 struct CellTape {
-  double h1, qxa, qya, n, qn, a, S, f, lim;
+  double h1, qxa, qya, n, qn, a, S, f, lim, ih;
   bool dry, fric, actx, acty, limx, limy, zerox, zeroy;
   double tempx, tempy;
 };
@@ -541,22 +575,23 @@ HB_HD C3 cell_fwd(const C3 &u, const C3 &r, double n, double dt, CellTape &tp) {
   }
   const double h = tp.h1;
   tp.n = n;
-  const double C_f = g * n * n * pow(h, -1.0 / 3.0);
   tp.qxa = u.qx + r.qx;
   tp.qya = u.qy + r.qy;
-  tp.qn = sqrt(tp.qxa * tp.qxa + tp.qya * tp.qya);
+  tp.qn = root(tp.qxa * tp.qxa + tp.qya * tp.qya);
   o.qx = tp.qxa;
   o.qy = tp.qya;
   if (!(n > 0.0)) return o;
   tp.fric = true;
-  tp.a = dt * C_f / (h * h);
-  tp.S = sqrt(1.0 + 4.0 * tp.a * tp.qn);
-  tp.f = 2.0 / (1.0 + tp.S);
-  tp.lim = 5.0 * h * sqrt(h * g);
+  // a = dt C_f / h^2, C_f = g n^2 h^(-1/3); the implicit value q (sqrt(1 + 4 a |q|)
+  // - 1) / (2 a |q|) as q f with f = 2 / (1 + S)
+  tp.ih = rcp(h);
+  tp.a = dt * g * n * n * inv_cbrt(h) * tp.ih * tp.ih;
+  tp.S = root(1.0 + 4.0 * tp.a * tp.qn);
+  tp.f = 2.0 * rcp(1.0 + tp.S);
+  tp.lim = 5.0 * h * root(h * g);
   if (fabs(tp.qxa) > 1.0e-10) {
     tp.actx = true;
-    const double temp = (1.0 - sqrt(1.0 + (4.0 * dt * C_f) / (h * h) * tp.qn)) /
-                        (-2.0 * dt * C_f / (h * h) * (tp.qn / tp.qxa));
+    const double temp = tp.qxa * tp.f;
     tp.tempx = temp;
     if (fabs(temp) > tp.lim) {
       tp.limx = true;
@@ -571,8 +606,7 @@ HB_HD C3 cell_fwd(const C3 &u, const C3 &r, double n, double dt, CellTape &tp) {
   }
   if (fabs(tp.qya) > 1.0e-10) {
     tp.acty = true;
-    const double temp = (1.0 - sqrt(1.0 + (4.0 * dt * C_f) / (h * h) * tp.qn)) /
-                        (-2.0 * dt * C_f / (h * h) * (tp.qn / tp.qya));
+    const double temp = tp.qya * tp.f;
     tp.tempy = temp;
     if (fabs(temp) > tp.lim) {
       tp.limy = true;
@@ -628,17 +662,18 @@ HB_HD void cell_rev(const CellTape &tp, const C3 &ob, double dt, C3 &ub, C3 &rb,
       const double f_b = tx_b * tp.qxa + ty_b * tp.qya;
       qxa_b += tx_b * tp.f;
       qya_b += ty_b * tp.f;
-      // f = 2/(1+S): df/dS = -2/(1+S)^2; S = sqrt(1 + 4 a qn): dS/d(a qn) = 2/S
-      const double x_b = f_b * (-2.0 / ((1.0 + tp.S) * (1.0 + tp.S))) * (2.0 / tp.S);
+      // f = 2/(1+S): df/dS = -2/(1+S)^2 = -f^2/2; S = sqrt(1 + 4 a qn): dS/d(a qn) = 2/S
+      const double x_b = -f_b * tp.f * tp.f * rcp(tp.S);
       const double a_b = x_b * tp.qn;
       const double qn_b = x_b * tp.a;
       if (tp.qn > 0.0) {
-        qxa_b += qn_b * tp.qxa / tp.qn;
-        qya_b += qn_b * tp.qya / tp.qn;
+        const double iqn = rcp(tp.qn);
+        qxa_b += qn_b * tp.qxa * iqn;
+        qya_b += qn_b * tp.qya * iqn;
       }
       // a = dt g n^2 h^(-7/3)
-      h1_b += a_b * tp.a * (-7.0 / 3.0) / tp.h1;
-      nb += a_b * tp.a * 2.0 / tp.n;
+      h1_b += a_b * tp.a * (-7.0 / 3.0) * tp.ih;
+      nb += a_b * tp.a * 2.0 * rcp(tp.n);
     }
   }
   (void)dt;

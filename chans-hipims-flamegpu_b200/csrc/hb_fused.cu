@@ -37,6 +37,7 @@
 
 #include "hb_common.cuh"
 #include "hb_datum_halo.cuh"
+#include "hb_fp64.cuh"
 #include "hb_once.h"
 #include "hb_physics.cuh"
 #include "hipims_b200_fused.h"

@@ -18,7 +18,7 @@
 //    faces east of lane 31 are evaluated by the first lanes of the same warp
 //    before the walk, one row a lane, so no warp waits for another);
 //  * reciprocals and square roots by one table-free cubic step from the
-//    hardware's approximate seed (rcp64, sqrt64: 3 and 6 FP64 operations
+//    hardware's approximate seed (hb_fp64.cuh: 3 and 6 FP64 operations
 //    instead of a division of about twelve and a root of about ten), one
 //    reciprocal per edge for both velocities, one for the wave span, dt / dx once
 //    per tile; the contact speed's sign is read off numerator and denominator;
@@ -43,27 +43,6 @@ __device__ __forceinline__ double sb(double a, double b) { return __dsub_rn(a, b
 __device__ __forceinline__ double mu(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double fm(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// 1 / x for normal x: the hardware's seed r0 (relative error e; 2^-19.9 at most
-// over 6e7 values of 2^-60..2^40) and the third-order iteration
-// r0 (1 + e + e^2) (Householder's method for 1/r - x), remainder e^3.  Largest
-// error over those values 2^-53 of the result.
-__device__ __forceinline__ double rcp64(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fm(-x, r, 1.0);
-  return fm(r, fm(e, e, e), r);
-}
-// sqrt(x) for x = 0 or normal x > 0: y0 ~ 1/sqrt(x) from the hardware, s0 = x y0,
-// e = 1 - s0 y0, and sqrt(x) = s0 (1 - e)^(-1/2) by its binomial series to e^2
-// (remainder 5/16 e^3).  Largest error over the same values 2^-52 of the result.
-__device__ __forceinline__ double sqrt64(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double s0 = mu(x, y);
-  const double e = fm(-s0, y, 1.0);
-  const double s = fm(mu(s0, e), fm(0.375, e, 0.5), s0);
-  return x > 0.0 ? s : 0.0;
-}
 __device__ __forceinline__ double max64(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ double min64(double a, double b) { return a < b ? a : b; }
 // max(x, 0) by the sign bit

@@ -99,7 +99,7 @@ class GaugeMisfit:
         self.nsteps, self.every, self.K = int(nsteps), int(every), int(checkpoint)
         self.weight = float(weight)
         self.h_reg = float(h_reg)
-        self.store_faces = bool(store_faces)
+        self.store_faces = bool(store_faces)  # no effect: every face is evaluated once per pass
         if forward_dtype not in (torch.float32, torch.float64):
             raise ValueError("forward_dtype must be float32 or float64")
         self.forward_dtype = forward_dtype
@@ -199,11 +199,6 @@ class GaugeMisfit:
         a.rows, a.cols, a.pitch, a.code_pitch = ins.rows, ins.cols, ins.pitch, ins.code_pitch
         a.mu, a.mu_stride, a.grad = mu.data_ptr(), n, grad.data_ptr()
         a.h_reg = self.h_reg
-        faces = None
-        if self.store_faces:  # each face's forward values once per reverse step
-            stride = (ins.rows + 1) * (ins.cols + 1)
-            faces = torch.empty(10 * stride, dtype=torch.float64, device=dev)
-            a.faces, a.face_stride = faces.data_ptr(), stride
         ctrlf = self.fs.ctrl.view(torch.float64)
         with torch.cuda.device(dev):
             for s0 in sorted(self._ckpt, reverse=True):
@@ -216,10 +211,10 @@ class GaugeMisfit:
                 self.fs.ctrl.copy_(ctrl)
                 self.fs.prepare()
                 for k in range(s0, s1):
-                    cur = self._state(k)
-                    for j in range(3):
-                        states[k - s0, j].copy_(cur[j])
-                    ctrl_log[k - s0].copy_(ctrlf[:_CTRL_DOUBLES])
+                    # state and clock of step k in one launch
+                    u = states[k - s0]
+                    torch._foreach_copy_([u[0], u[1], u[2], ctrl_log[k - s0]],
+                                         [*self._state(k), ctrlf[:_CTRL_DOUBLES]])
                     if k + 1 < s1:
                         self.fs.step(1)
                 log = ctrl_log[: s1 - s0].cpu().numpy()
