@@ -515,6 +515,91 @@ infiltration_kernel(int64_t M, const int32_t *__restrict__ wet, T *__restrict__ 
   hu[i] -= dF;
 }
 
+// Ordered list of the cells that pass a test, as torch.nonzero gives it, in two
+// kernels: a block tests kListCells cells, keeps their bits and counts them;
+// then each block adds up the counts before its own and writes its ids.  Bound
+// by the reads of h (and the neighbour table); against the mask, its fill, the
+// comparison kernels, the three kernels of nonzero and the cast to int32 it is
+// two launches instead of nine: a step of the solver object on 256 x 300 cells
+// (FP32, host-bound) 349 -> 279 us, 241 with the raw stream handle.
+constexpr int kListCells = 4096, kListThreads = 256, kListWords = kListCells / 32;
+
+// RULE 0: fluxMask (HC/fluxMaskGenerator_Kernel.cu:19-42; x = t); 1: the update
+// list of HP/SWE_CUDA.py:786-790, |h_update| > 0 or h >= 0 (x = h_update).
+template <typename T, int RULE>
+__global__ void __launch_bounds__(kListThreads)
+list_test_kernel(int64_t N, const T *__restrict__ h, const int32_t *__restrict__ index,
+                 const T *__restrict__ x, uint32_t *__restrict__ words,
+                 int32_t *__restrict__ counts) {
+  __shared__ int s_n;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  const T hs = T(kHSmall);
+  const bool first = RULE == 0 && x[0] == T(0);
+  int mine = 0;
+#pragma unroll 4
+  for (int k = 0; k < kListCells / kListThreads; k++) {
+    const int64_t i = (int64_t)blockIdx.x * kListCells + k * kListThreads + threadIdx.x;
+    bool m = false;
+    if (i < N) {
+      if constexpr (RULE == 0) {
+        m = first || h[i] > hs;
+        if (!m) {
+#pragma unroll
+          for (int nei = 1; nei < 5; nei++) {
+            const int32_t q = index[(int64_t)nei * N + i];
+            if (q > 0) m = m || (h[q] > hs);  // cell 0 never activates its neighbours
+          }
+        }
+      } else {
+        m = fabs(x[i]) > T(0) || h[i] >= T(0);
+      }
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) {
+      words[(int64_t)blockIdx.x * kListWords + (k * kListThreads + threadIdx.x) / 32] = b;
+      mine += __popc(b);
+    }
+  }
+  if ((threadIdx.x & 31) == 0) atomicAdd(&s_n, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) counts[blockIdx.x] = s_n;
+}
+
+__global__ void __launch_bounds__(kListThreads)
+list_write_kernel(const uint32_t *__restrict__ words, const int32_t *__restrict__ counts,
+                  int32_t *__restrict__ list, int32_t *__restrict__ total) {
+  __shared__ int s_red[kListThreads / 32], s_pos[kListWords];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  int before = 0;
+  for (int b = tid; b < (int)blockIdx.x; b += kListThreads) before += counts[b];
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  if (lane == 0) s_red[w] = before;
+  // exclusive scan of the block's words
+  const uint32_t *bw = words + (int64_t)blockIdx.x * kListWords;
+  int c = tid < kListWords ? __popc(bw[tid]) : 0, inc = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  __shared__ int s_warp[kListThreads / 32];
+  if (lane == 31) s_warp[w] = inc;
+  __syncthreads();
+  int base = 0;
+  for (int q = 0; q < kListThreads / 32; q++) base += s_red[q];
+  int pos = base + inc - c;
+  for (int q = 0; q < w; q++) pos += s_warp[q];
+  if (tid < kListWords) s_pos[tid] = pos;
+  __syncthreads();
+  for (int k = w; k < kListWords; k += kListThreads / 32) {
+    const uint32_t bits = bw[k];
+    if ((bits >> lane) & 1u)
+      list[s_pos[k] + __popc(bits & ((1u << lane) - 1u))] =
+          (int32_t)((int64_t)blockIdx.x * kListCells + k * 32 + lane);
+  }
+  if (blockIdx.x == gridDim.x - 1 && tid == 0) *total = base + counts[blockIdx.x];
+}
+
 // Two-level min: blocks reduce to partials, the last block to finish reduces
 // the partials (counter-based, no spinning).
 constexpr int kMinThreads = 1024;
@@ -626,6 +711,35 @@ extern "C" int hb_flux_mask(int dtype, int64_t N, uint8_t *flux_mask, const void
     flux_mask_kernel<float><<<blocks_for(N, kThreads), kThreads, 0, s>>>(
         N, flux_mask, (const float *)h, index, (const float *)t);
   return check_launch("hb_flux_mask");
+}
+
+extern "C" size_t hb_cell_list_workspace_size(int64_t N) {
+  const int64_t nb = (N + kListCells - 1) / kListCells;
+  return N <= 0 ? 0 : (size_t)nb * (kListWords + 1) * sizeof(uint32_t);
+}
+
+extern "C" int hb_cell_list(int dtype, int rule, int64_t N, const void *h, const int32_t *index,
+                            const void *x, int32_t *list, int32_t *count, void *workspace,
+                            void *stream) {
+  HB_REQUIRE(!bad_dtype(dtype), "hb_cell_list: bad dtype %d", dtype);
+  HB_REQUIRE(rule == 0 || rule == 1, "hb_cell_list: rule must be 0 or 1 (got %d)", rule);
+  HB_REQUIRE(N > 0 && N <= INT32_MAX, "hb_cell_list: bad N=%lld", (long long)N);
+  HB_REQUIRE(h && x && list && count && workspace && (rule != 0 || index),
+             "hb_cell_list: null pointer");
+  auto s = as_stream(stream);
+  const unsigned nb = (unsigned)((N + kListCells - 1) / kListCells);
+  uint32_t *words = (uint32_t *)workspace;
+  int32_t *counts = (int32_t *)(words + (size_t)nb * kListWords);
+#define HB_LIST_TEST(T, R) \
+  list_test_kernel<T, R><<<nb, kListThreads, 0, s>>>(N, (const T *)h, index, (const T *)x, words, counts)
+  if (dtype == HB_F64) {
+    if (rule == 0) HB_LIST_TEST(double, 0); else HB_LIST_TEST(double, 1);
+  } else {
+    if (rule == 0) HB_LIST_TEST(float, 0); else HB_LIST_TEST(float, 1);
+  }
+#undef HB_LIST_TEST
+  list_write_kernel<<<nb, kListThreads, 0, s>>>(words, counts, list, count);
+  return check_launch("hb_cell_list");
 }
 
 extern "C" int hb_flux(int order, int dtype, int64_t M, int64_t N, const int32_t *wet_mask,

@@ -102,6 +102,8 @@ SIGNATURES = {
     "hb_last_error": (ctypes.c_char_p, []),
     "hb_record_sizes": (None, [ctypes.POINTER(ctypes.c_size_t)]),
     "hb_flux_mask": (_I, [_I, _L, _P, _P, _P, _P, _P]),
+    "hb_cell_list_workspace_size": (ctypes.c_size_t, [_L]),
+    "hb_cell_list": (_I, [_I, _I, _L, _P, _P, _P, _P, _P, _P, _P]),
     "hb_flux": (_I, [_I, _I, _L, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I,
                      _P, _I, _I, _P, _I, _I, _P, _P, _P, _P]),
     "hb_friction_update": (_I, [_I, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,

@@ -18,6 +18,7 @@ are checked and CUDA launch errors raise instead of being printed.
 """
 from __future__ import annotations
 
+import contextlib
 import threading
 
 import torch
@@ -58,7 +59,19 @@ def _p(x: torch.Tensor) -> int:
 
 
 def _stream(x: torch.Tensor) -> int:
-    return torch.cuda.current_stream(x.device).cuda_stream
+    # the raw handle: torch.cuda.current_stream() builds a Stream object, some
+    # 5 us on each of a step's eight calls
+    return torch._C._cuda_getCurrentRawStream(x.device.index)
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _on(x: torch.Tensor):
+    """Context with x's device current (nothing to do where it already is)."""
+    if torch.cuda.current_device() == x.device.index:
+        return _SAME_DEVICE
+    return torch.cuda.device(x.device)
 
 
 def _table(x: torch.Tensor) -> tuple[int, int]:
@@ -86,7 +99,7 @@ def _flux(order: int, wetMask, h_flux, qx_flux, qy_flux, h, wl, z, qx, qy, index
     wr, wc = _table(given_wl)
     qr, qc = _table(given_q)
     L = _lib.lib()
-    with torch.cuda.device(h.device):
+    with _on(h):
         rc = L.hb_flux(order, dtype, M, N, _p(wetMask), _p(h_flux), _p(qx_flux), _p(qy_flux),
                        _p(h), _p(wl), _p(z), _p(qx), _p(qy), _p(index), _p(normal),
                        _p(given_depth), dr, dc, _p(given_wl), wr, wc, _p(given_q), qr, qc,
@@ -120,7 +133,7 @@ def friction_update(wetMask, h_update, qx_update, qy_update, z_update, landuse, 
     _need("wetMask", wetMask, torch.int32)
     _need("landuse", landuse, torch.uint8)
     L = _lib.lib()
-    with torch.cuda.device(h.device):
+    with _on(h):
         rc = L.hb_friction_update(dtype, wetMask.numel(), _p(wetMask), _p(h_update),
                                   _p(qx_update), _p(qy_update), _p(z_update), _p(landuse),
                                   _p(h), _p(wl), _p(qx), _p(qy), _p(z), _p(manning), _p(dt),
@@ -138,7 +151,7 @@ def update_timestep(wetMask, accelerator, h_max, h, qx, qy, dx, CFL, t, dt) -> N
     if accelerator.numel() < wetMask.numel():
         raise RuntimeError("accelerator must hold one entry per listed cell")
     L = _lib.lib()
-    with torch.cuda.device(h.device):
+    with _on(h):
         rc = L.hb_timestep(dtype, wetMask.numel(), _p(wetMask), _p(accelerator), _p(h_max),
                            _p(h), _p(qx), _p(qy), _p(dx), _p(CFL), _p(t), _p(dt), _stream(h))
     _lib.check(rc, "updateTimestep")
@@ -151,7 +164,7 @@ def station_rain(h_update, rainStationMask, rainStationData, dt) -> None:
     dtype = _dtype_of(h_update, dict(rainStationData=rainStationData, dt=dt))
     _need("rainStationMask", rainStationMask, torch.int16)
     L = _lib.lib()
-    with torch.cuda.device(h_update.device):
+    with _on(h_update):
         rc = L.hb_rain_station(dtype, rainStationMask.numel(), _p(h_update),
                                _p(rainStationMask), _p(rainStationData), _p(dt),
                                _stream(h_update))
@@ -166,10 +179,44 @@ def flux_mask(fluxMask, h, index, t) -> None:
         raise RuntimeError("fluxMask must be bool")
     _need("index", index, torch.int32)
     L = _lib.lib()
-    with torch.cuda.device(h.device):
+    with _on(h):
         rc = L.hb_flux_mask(dtype, h.numel(), _p(fluxMask), _p(h), _p(index), _p(t),
                             _stream(h))
     _lib.check(rc, "fluxMask.update")
+
+
+def _cell_list(rule: int, h: torch.Tensor, index, x: torch.Tensor) -> torch.Tensor:
+    dtype = _dtype_of(h, dict(x=x))
+    n = h.numel()
+    if n == 0:
+        return torch.empty(0, dtype=torch.int32, device=h.device)
+    L = _lib.lib()
+    words = (L.hb_cell_list_workspace_size(n) + 3) // 4
+    buf = torch.empty(n + 1 + words, dtype=torch.int32, device=h.device)
+    with _on(h):
+        rc = L.hb_cell_list(dtype, rule, n, _p(h), None if index is None else _p(index), _p(x),
+                            _p(buf), _p(buf) + 4 * n, _p(buf) + 4 * (n + 1), _stream(h))
+        _lib.check(rc, "cell list")
+        return buf[: buf[n].item()]
+
+
+def active_list(h, index, t) -> torch.Tensor:
+    """Ids (int32, ascending) of the cells fluxMask.update marks: the list
+    nonzero() makes of the mask."""
+    _check(dict(h=h, index=index, t=t))
+    _need("index", index, torch.int32)
+    if index.numel() != 5 * h.numel():
+        raise RuntimeError(f"index must hold 5*N = {5 * h.numel()} entries (got {index.numel()})")
+    return _cell_list(0, h, index, t)
+
+
+def update_list(h_update, h) -> torch.Tensor:
+    """Ids (int32, ascending) of the cells with |h_update| > 0 or h >= 0
+    (HP/SWE_CUDA.py:786-790)."""
+    _check(dict(h_update=h_update, h=h))
+    if h_update.numel() != h.numel():
+        raise RuntimeError("h_update and h must have one entry per cell")
+    return _cell_list(1, h, None, h_update)
 
 
 def euler_update(updateMask, h_update, qx_update, qy_update, z_update, h, wl, z, qx,
@@ -181,7 +228,7 @@ def euler_update(updateMask, h_update, qx_update, qy_update, z_update, h, wl, z,
                               z_update=z_update, wl=wl, z=z, qx=qx, qy=qy))
     _need("updateMask", updateMask, torch.int32)
     L = _lib.lib()
-    with torch.cuda.device(h.device):
+    with _on(h):
         rc = L.hb_euler_update(dtype, updateMask.numel(), _p(updateMask), _p(h_update),
                                _p(qx_update), _p(qy_update), _p(z_update), _p(h), _p(wl),
                                _p(z), _p(qx), _p(qy), _stream(h))
@@ -202,7 +249,7 @@ def infiltration(wetMask, h_update, landuse, h, hydraulic_conductivity, capillar
     _need("wetMask", wetMask, torch.int32)
     _need("landuse", landuse, torch.uint8)
     L = _lib.lib()
-    with torch.cuda.device(h.device):
+    with _on(h):
         rc = L.hb_infiltration(dtype, wetMask.numel(), _p(wetMask), _p(h_update), _p(landuse),
                                _p(h), _p(hydraulic_conductivity), _p(capillary_head),
                                _p(water_content_diff), _p(cumulative_depth), _p(dt),
@@ -239,7 +286,7 @@ def device_min(x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor
     L = _lib.lib()
     nbytes = L.hb_min_reduce_workspace_size(x.numel())
     ws = _min_workspace(x, nbytes) if nbytes else None
-    with torch.cuda.device(x.device):
+    with _on(x):
         rc = L.hb_min_reduce(dtype, x.numel(), _p(x), _p(out), _p(ws) if ws is not None else None,
                              _stream(x))
     _lib.check(rc, "device_min")
@@ -261,7 +308,7 @@ def gather(cell_offsets: torch.Tensor, h: torch.Tensor, qx: torch.Tensor | None 
         ou = torch.empty_like(oh)
         ov = torch.empty_like(oh)
     L = _lib.lib()
-    with torch.cuda.device(h.device):
+    with _on(h):
         rc = L.hb_gather(dtype, n, _p(cell_offsets), _p(h),
                          _p(qx) if qx is not None else None, _p(qy) if qy is not None else None,
                          _p(oh), _p(ou) if ou is not None else None,

@@ -128,9 +128,12 @@ class Godunov:
     # ------------------------------------------------------------------ step
     def addFlux(self):
         """fluxMask -> active list -> HLLC flux accumulation (HP/SWE_CUDA.py:339-424)."""
-        fm = torch.zeros_like(self._h_internal, dtype=torch.bool)
-        self._ops.flux_mask(fm, self._h_internal, self._index, self.t)
-        self._wetMask = torch.flatten(fm.nonzero()).to(torch.int32)
+        if self._ops is ops:
+            self._wetMask = ops.active_list(self._h_internal, self._index, self.t)
+        else:
+            fm = torch.zeros_like(self._h_internal, dtype=torch.bool)
+            self._ops.flux_mask(fm, self._h_internal, self._index, self.t)
+            self._wetMask = torch.flatten(fm.nonzero()).to(torch.int32)
         op = self._ops.flux_2nd_order if self._secondOrder else self._ops.flux_1st_order
         op(self._wetMask, self._h_update, self._qx_update, self._qy_update, self._h_internal,
            self._wl_internal, self._z_internal, self._qx_internal, self._qy_internal,
@@ -169,6 +172,8 @@ class Godunov:
         self._h_update += rainfall_raster * self.dt
 
     def _update_list(self) -> torch.Tensor:
+        if self._ops is ops:
+            return ops.update_list(self._h_update, self._h_internal)
         return torch.flatten(((self._h_update.abs() > 0.0) | (self._h_internal >= 0.0))
                              .nonzero()).to(torch.int32)
 
@@ -178,6 +183,14 @@ class Godunov:
                                   self._qy_update, self._z_update, self._landuseMask,
                                   self._h_internal, self._wl_internal, self._qx_internal,
                                   self._qy_internal, self._z_internal, self._manning, self.dt)
+
+    def _time_steps(self) -> torch.Tensor:
+        """The per-cell time steps of the listed cells, to be written by update_timestep."""
+        if self._ops is ops:  # writes every listed entry
+            return torch.empty(self._wetMask.size(), dtype=self._tensorType,
+                               device=self._wetMask.device)
+        return torch.full(self._wetMask.size(), self._maxTimeStep.item(),
+                          dtype=self._tensorType, device=self._wetMask.device)
 
     def _advance_dt(self, time_upper: torch.Tensor, listed: int) -> None:
         """min -> 10x cap -> export clip -> t += dt (HP/SWE_CUDA.py:818-831)."""
@@ -194,8 +207,7 @@ class Godunov:
     def time_friction_euler_update_cuda(self, device):
         time_upper = self.dt * 10.0
         self.friction_euler_update_cuda()
-        self._accelerator_dt = torch.full(self._wetMask.size(), self._maxTimeStep.item(),
-                                          dtype=self._tensorType, device=device)
+        self._accelerator_dt = self._time_steps()
         self._ops.update_timestep(self._wetMask, self._accelerator_dt, self._h_max,
                                   self._h_internal, self._qx_internal, self._qy_internal,
                                   self.dx, self.cfl, self.t, self.dt)
@@ -216,8 +228,7 @@ class Godunov:
     def time_update_cuda(self, device):
         time_upper = self.dt * 10.0
         self._wetMask = torch.flatten((self._h_internal > 1.0e-6).nonzero()).to(torch.int32)
-        self._accelerator_dt = torch.full(self._wetMask.size(), self._maxTimeStep.item(),
-                                          dtype=self._tensorType, device=device)
+        self._accelerator_dt = self._time_steps()
         self._ops.update_timestep(self._wetMask, self._accelerator_dt, self._h_max,
                                   self._h_internal, self._qx_internal, self._qy_internal,
                                   self.dx, self.cfl, self.t, self.dt)

@@ -56,6 +56,20 @@ void hb_record_sizes(size_t out[3]);
 int hb_flux_mask(int dtype, int64_t N, uint8_t *flux_mask, const void *h,
                  const int32_t *index, const void *t, void *stream);
 
+/* ======================================================================
+ * Cell lists of a step (no single reference op): the ascending ids of the
+ * cells that pass a test, list[N] (int32), and their number, count[1], in
+ * device memory.
+ *   rule 0: the fluxMask test, x = t [1] (HP/SWE_CUDA.py:339-352: fluxMask,
+ *           nonzero, int32)
+ *   rule 1: |x| > 0 or h >= 0, x = h_update [N] (HP/SWE_CUDA.py:786-790)
+ * workspace: hb_cell_list_workspace_size(N) bytes.
+ * ==================================================================== */
+size_t hb_cell_list_workspace_size(int64_t N);
+int hb_cell_list(int dtype, int rule, int64_t N, const void *h, const int32_t *index,
+                 const void *x, int32_t *list, int32_t *count, void *workspace,
+                 void *stream);
+
 /* fluxCal_2ndOrder_jh_improved.addFlux (order = 2,
  * HC/fluxCal_2ndOrder_jh_improved.cpp:28-53) and
  * fluxCalculation_jh_modified_surface.addFlux (order = 1,
