@@ -592,7 +592,24 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
   }
   const int bug_y = in.bug_y, bug_x = in.bug_x;
   float datum_tile = 0.f;
-  if (in.datum && !skip) {
+  // all-valid tiles: the shift of the halo beds this warp reads into the tile's
+  // datum (warp 0: rows -2, -1 and, before the walk, columns 64, 65; warp 1:
+  // columns -2, -1; warp 3: rows TY, TY + 1)
+  float dz_row = 0.f, dz_col = 0.f;
+  if (ALLV && in.datum) {
+    const int by = y0 / HB_DATUM_BLOCK, bx = x0 / HB_DATUM_BLOCK;
+    const float *d = in.datum + by * in.datum_nx + bx;
+    const float own = d[0];
+    if (w == 0) {
+      if (y0 % HB_DATUM_BLOCK == 0 && by > 0) dz_row = d[-in.datum_nx] - own;
+      if (bx + 1 < in.datum_nx) dz_col = d[1] - own;
+    } else if (w == 1) {
+      if (bx > 0) dz_col = d[-1] - own;
+    } else if (w == kRowsNW - 1) {
+      if ((y0 + TY) % HB_DATUM_BLOCK == 0 && by + 1 < in.datum_ny) dz_row = d[in.datum_nx] - own;
+    }
+  }
+  if (!ALLV && in.datum && !skip) {
     const int by = y0 / HB_DATUM_BLOCK, bx = x0 / HB_DATUM_BLOCK;
     datum_tile = in.datum[by * in.datum_nx + bx];
     if (tid >= 32 && tid < 41) {
@@ -626,8 +643,7 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
       if (lane == 0) s.rowmask = m;
     }
   }
-  if (in.datum && !skip) {
-    __syncthreads();  // ddatum visible
+  if (!ALLV && in.datum && !skip) {
     const int by0 = (y0 / HB_DATUM_BLOCK) * HB_DATUM_BLOCK;
     const int bx0 = (x0 / HB_DATUM_BLOCK) * HB_DATUM_BLOCK;
     const DatumHalo dh = datum_halo(y0, x0, by0, bx0, TY, kPW, kPSWF, HB_DATUM_BLOCK);
@@ -641,7 +657,18 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
       if (dyb != 1 || dxb != 1) s.f[3][V.fi(i, j)] += s.ddatum[dyb * 3 + dxb];
     }
   }
-  __syncthreads();
+  if constexpr (!ALLV) __syncthreads();  // beds and rowmask
+  // All-valid tiles: every halo bed has one reader before the next barrier, the
+  // lane that shifts it (rows: the lane's own columns; columns: the rows whose
+  // edge this lane prepares below), so no pass and no barrier of its own is
+  // needed.
+  if (ALLV && dz_row != 0.f) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      f2 *zr = reinterpret_cast<f2 *>(&s.f[3][V.fi(w == 0 ? -2 + q : TY + q, 2 * lane)]);
+      *zr = add2(*zr, dup(dz_row));
+    }
+  }
 
   // --- tile edges: warp 0 the faces between columns 63 | 64 (east faces of
   // lane 31's second cell), two rows per lane; warp 1 the x-slopes of
@@ -649,6 +676,10 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
   if (skip) {
   } else if (w == 0) {
     for (int i = 2 * lane; i < TY; i += 64) {
+      if (ALLV && dz_col != 0.f) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) s.f[3][V.fi(i + (q >> 1), kPW + (q & 1))] += dz_col;
+      }
       float a[4], b[4];  // slopes of col 63 / col 64 for rows i, i + 1 (h, z, qx, qy)
       float a1[4], b1[4];
       xslope1<TY, ALLV>(V, i, 63, a[0], a[1], a[2], a[3]);
@@ -666,6 +697,10 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
     }
   } else if (w == 1) {
     for (int i = lane; i < TY; i += 32) {
+      if (ALLV && dz_col != 0.f) {
+        s.f[3][V.fi(i, -2)] += dz_col;
+        s.f[3][V.fi(i, -1)] += dz_col;
+      }
       float sh, sz, sqx, sqy;
       xslope1<TY, ALLV>(V, i, -1, sh, sz, sqx, sqy);
       s.sxw[i][1] = sz;
