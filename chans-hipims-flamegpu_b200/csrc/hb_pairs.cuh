@@ -225,36 +225,28 @@ __device__ __forceinline__ void face_core2(f2 ah, f2 bh, f2 bz, f2 Lh, f2 Lz0, f
   const f2 nfR = fma2(uR, qnR, mul2(mul2(dup(kHalfGF), hR), hR));
   const f2 pR = mul2(hR, sub2(uR, sR)), pL = mul2(hL, sub2(uL, sL));
   const f2 num = sub2(mul2(sL, pR), mul2(sR, pL)), den = sub2(pR, pL);
-  const f2 sM = mul2(num, pk(rcpa(den.x), rcpa(den.y)));
-  const f2 dS = sub2(sR, sL);
-  const f2 inv = pk(rcpa(dS.x), rcpa(dS.y));
-  const f2 sLR = mul2(sL, sR);
-  const f2 hfM = mul2(fma2(sLR, sub2(hR, hL), sub2(mul2(sR, hfL), mul2(sL, hfR))), inv);
-  f2 vU;
-  const f2 nfM = mul2(fma2(sLR, sub2(qnR, qnL), sub2(mul2(sR, nfL), mul2(sL, nfR))), inv);
-#pragma unroll
-  for (int c = 0; c < 2; c++) {
-    const float sl = c ? sL.y : sL.x, sr = c ? sR.y : sR.x, sm = c ? sM.y : sM.x;
-    // the reference's chain sL >= 0 / sL < 0 <= sM / sM < 0 <= sR / else,
-    // with sL finite (it is, for a finite state)
-    const bool left = 0.f <= sl;
-    const bool midL = !left && 0.f <= sm;
-    const bool midR = !left && sm < 0.f && 0.f <= sr;
-    const bool mid = midL || midR;
-    const bool dry = ((c ? hL.y : hL.x) < kHsF && (c ? hR.y : hR.x) < kHsF) || (c ? dd1 : dd0);
-    float h_ = left ? (c ? hfL.y : hfL.x) : (mid ? (c ? hfM.y : hfM.x) : (c ? hfR.y : hfR.x));
-    float n_ = left ? (c ? nfL.y : nfL.x) : (mid ? (c ? nfM.y : nfM.x) : (c ? nfR.y : nfR.x));
-    if (dry) h_ = n_ = 0.f;
-    // the tangential flux is the mass flux times the upwind side's
-    // tangential velocity in every region (the reference forms the
-    // unstarred ones as u * (v * h); (u * h) * v here: one rounding apart)
-    const float vu = (left || midL) ? (c ? vL.y : vL.x) : (c ? vR.y : vR.x);
-    if (c) {
-      fh.y = h_; fn.y = n_; vU.y = vu;
-    } else {
-      fh.x = h_; fn.x = n_; vU.x = vu;
-    }
-  }
+  // only the contact speed's sign is used: that of num / den is num * den's
+  const f2 sM = mul2(num, den);
+  // The star flux with the wave speeds clamped at 0 is the flux of every region:
+  // at sL >= 0 it is FL (sR / sR) and at sR <= 0 FR (sL / sL), equal to the unstarred
+  // fluxes up to the rounding of one reciprocal, and in between it is the star
+  // flux itself.  A face between dry sides has the factor 0.  (Selecting the
+  // region's fluxes took seven more instructions per face: 84.0 us a step on
+  // 2048^2, 79.9 so.)
+  const f2 cL = pk(fminf(sL.x, 0.f), fminf(sL.y, 0.f));
+  const f2 cR = pk(fmaxf(sR.x, 0.f), fmaxf(sR.y, 0.f));
+  const f2 dS = sub2(cR, cL);
+  const bool dry0 = (hL.x < kHsF && hR.x < kHsF) || dd0;
+  const bool dry1 = (hL.y < kHsF && hR.y < kHsF) || dd1;
+  const f2 inv = pk(dry0 ? 0.f : rcpa(dS.x), dry1 ? 0.f : rcpa(dS.y));
+  const f2 cLR = mul2(cL, cR);
+  fh = mul2(fma2(cLR, sub2(hR, hL), sub2(mul2(cR, hfL), mul2(cL, hfR))), inv);
+  fn = mul2(fma2(cLR, sub2(qnR, qnL), sub2(mul2(cR, nfL), mul2(cL, nfR))), inv);
+  // the tangential flux is the mass flux times the upwind side's tangential
+  // velocity in every region (the reference forms the unstarred ones as
+  // u * (v * h); (u * h) * v here: one rounding apart)
+  const f2 vU = pk(0.f <= sL.x || 0.f <= sM.x ? vL.x : vR.x,
+                   0.f <= sL.y || 0.f <= sM.y ? vL.y : vR.y);
   ft = mul2(fh, vU);
 }
 
