@@ -110,25 +110,23 @@ __device__ __forceinline__ void face_core64(double Ah, double Az, double Bh, dou
   const double sR = thinR ? fm(2.0, aL, uL) : max64(ad(uR, aR), ad(us, as));
   const double nL = fm(uL, qL, mu(mu(0.5, gL), hL)), nR = fm(uR, qR, mu(mu(0.5, gR), hR));
   const double pL = mu(hL, sb(uL, sL)), pR = mu(hR, sb(uR, sR));
-  // contact speed sM = num / den: only its sign is needed (den = 0: neither)
+  // contact speed sM = num / den: only its sign is needed (den != 0 where a side
+  // is wet)
   const double num = sb(mu(sL, pR), mu(sR, pL)), den = sb(pR, pL);
-  const int sg = __double2hiint(num) ^ __double2hiint(den);
-  const bool zero = num == 0.0;
-  const bool some = den != 0.0;
-  const bool left = 0.0 <= sL;
-  const bool midL = !left && some && (sg >= 0 || zero);
-  const bool midR = !left && some && !(sg >= 0 || zero) && 0.0 <= sR;
-  const bool mid = midL || midR;
-  const double inv = rcp64(sb(sR, sL)), sLR = mu(sL, sR);
-  const double hM = mu(fm(sLR, sb(hR, hL), sb(mu(sR, qL), mu(sL, qR))), inv);
-  const double nM = mu(fm(sLR, sb(qR, qL), sb(mu(sR, nL), mu(sL, nR))), inv);
-  const bool none = hL < hs && hR < hs;
+  const bool up = 0.0 <= sL || num == 0.0 ||
+                  (__double2hiint(num) ^ __double2hiint(den)) >= 0;
+  // The star flux with the wave speeds clamped at 0 is the flux of every region
+  // (at sL >= 0 it is FL (sR / sR), at sR <= 0 FR), up to the rounding of one
+  // reciprocal; a face between dry sides has the factor 0
   const bool dd = dryA && dryB;
-  fh = left ? qL : (mid ? hM : qR);
-  fn = left ? nL : (mid ? nM : nR);
-  if (none || dd) fh = fn = 0.0;
+  const double cL = __double2hiint(sL) < 0 ? sL : 0.0, cR = pos64(sR);
+  double inv = rcp64(sb(cR, cL));
+  if ((hL < hs && hR < hs) || dd) inv = 0.0;
+  const double cLR = mu(cL, cR);
+  fh = mu(fm(cLR, sb(hR, hL), sb(mu(cR, qL), mu(cL, qR))), inv);
+  fn = mu(fm(cLR, sb(qR, qL), sb(mu(cR, nL), mu(cL, nR))), inv);
   // the tangential flux is the mass flux times the upwind tangential velocity
-  ft = mu(fh, (left || midL) ? vL : vR);
+  ft = mu(fh, up ? vL : vR);
   if (dd) sa = sbt = 0.0;
 }
 
