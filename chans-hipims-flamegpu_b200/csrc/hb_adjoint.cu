@@ -26,6 +26,8 @@ static_assert(sizeof(hb_adjoint_args) == 184, "hb_adjoint_args layout (ctypes mi
 namespace hb {
 namespace {
 
+#include "hb_face64.cuh"
+
 using namespace adj;
 
 struct Grid {
@@ -87,21 +89,19 @@ __device__ void load_bc(const hb_instance &in, double t, BcVals &bc) {
 }
 
 // Face (A at (ra, ca) minus side, B at (rb, cb) plus side) along DIR, any
-// validity.  Forward only when bar == nullptr; otherwise reverse with the
-// output adjoint `ob` and scatter into lam (atomics).
+// validity, reversed with the output adjoint `ob` and scattered into lam
+// (atomics).
 template <int DIR>
-__device__ FaceOut5 face_at(const Grid &G, const BcVals &bc, int ra, int ca, int rb, int cb,
-                            const FaceOut5 *ob, double *lh, double *lqx, double *lqy,
-                            double hreg = 0.0) {
+__device__ void face_at(const Grid &G, const BcVals &bc, int ra, int ca, int rb, int cb,
+                        const FaceOut5 &ob, double *lh, double *lqx, double *lqy, double hreg) {
   const int dr = rb - ra, dc = cb - ca;  // unit step from A to B
   const bool va = G.valid(ra, ca), vb = G.valid(rb, cb);
-  FaceOut5 o{0, 0, 0, 0, 0};
-  if (!va && !vb) return o;
+  if (!va && !vb) return;
   FaceIn fi;
   FaceTape<DIR> tp;
   int rL = ra - dr, cL = ca - dc, rR = rb + dr, cR = cb + dc;
   double jac[3] = {1, 1, 1};
-  bool ghostA = false, ghostB = false;
+  bool ghostA = false;
   if (va && vb) {
     fi.A = G.cell(ra, ca);
     fi.B = G.cell(rb, cb);
@@ -118,7 +118,7 @@ __device__ FaceOut5 face_at(const Grid &G, const BcVals &bc, int ra, int ca, int
     Cz Gh;
     if (!ghost_of(bc.type[cls], DIR, C, bc.v[cls][0], bc.v[cls][1], bc.v[cls][2],
                   bc.v[cls][3], Gh, jac))
-      return o;
+      return;
     fi.A = va ? C : Gh;
     fi.B = va ? Gh : C;
     fi.L = fi.A;
@@ -126,25 +126,23 @@ __device__ FaceOut5 face_at(const Grid &G, const BcVals &bc, int ra, int ca, int
     fi.vL = fi.vR = false;
     fi.noslope = true;
     ghostA = !va;
-    ghostB = !vb;
   }
-  o = face_fwd<DIR>(fi, tp);
-  if (!ob) return o;
+  face_fwd<DIR>(fi, tp);
   FaceBar xb{};
-  face_rev<DIR>(fi, tp, *ob, xb);
-  auto add = [&](int r, int c, const C3 &v) {
-    if (!G.valid(r, c)) return;
+  face_rev<DIR>(fi, tp, ob, xb);
+  // into a valid cell of depth h (a masked cell's state adjoint stays zero)
+  auto add = [&](int r, int c, double h, const C3 &v) {
+    if (h < hreg) return;
     const size_t k = G.off(r, c);
-    if (G.h[k] < hreg) return;  // masked cell: its state adjoint stays zero
     if (v.h != 0.0) atomicAdd(lh + k, v.h);
     if (v.qx != 0.0) atomicAdd(lqx + k, v.qx);
     if (v.qy != 0.0) atomicAdd(lqy + k, v.qy);
   };
   if (va && vb) {
-    add(rL, cL, xb.L);
-    add(ra, ca, xb.A);
-    add(rb, cb, xb.B);
-    add(rR, cR, xb.R);
+    if (fi.vL) add(rL, cL, fi.L.h, xb.L);
+    add(ra, ca, fi.A.h, xb.A);
+    add(rb, cb, fi.B.h, xb.B);
+    if (fi.vR) add(rR, cR, fi.R.h, xb.R);
   } else {
     // only the valid cell receives: directly, and through its ghost
     C3 c = ghostA ? xb.B : xb.A;
@@ -152,30 +150,52 @@ __device__ FaceOut5 face_at(const Grid &G, const BcVals &bc, int ra, int ca, int
     c.h += gb.h * jac[0];
     c.qx += gb.qx * jac[1];
     c.qy += gb.qy * jac[2];
-    add(va ? ra : rb, va ? ca : cb, c);
+    add(va ? ra : rb, va ? ca : cb, va ? fi.A.h : fi.B.h, c);
   }
-  return o;
 }
 
-// Whether the face between (ra, ca) and (rb, cb) needs the boundary tables
-// (exactly one valid side).
-__device__ __forceinline__ bool is_ghost_face(const Grid &G, int ra, int ca, int rb, int cb) {
-  return G.valid(ra, ca) != G.valid(rb, cb);
-}
-
-// Pass 1: a block of 32 x 8 cells and nine warps.  Each face of the block's
-// cells is evaluated once into shared memory (warps 0-7: the west and north
-// faces of their row's cells; warp 8: the last row of y-faces and the last
-// column of x-faces), then the cells are updated and reversed.  FP64 issue and
-// latency bind it (45 % of issue slots).  With the faces in a pass of their own
-// through global memory, IEEE divisions, pow and the boundary tables searched by
-// every block, the two passes took 27 + 41 us (512^2 cells, cold); 34 us so.
+// Forward values of the face between (ra, ca) (minus side) and (rb, cb): the
+// step's own face (hb_face64.cuh), cells by their place in the staged tile.
 constexpr int kCellRows = 8;
-__global__ void __launch_bounds__(32 * (kCellRows + 1), 2)
+constexpr int kTileRows = kCellRows + 4, kTileCols = 32 + 4;
+struct CellTile {  // a block's cells and two around them: h, qx, qy, z and codes
+  double f[4][kTileRows][kTileCols];
+  uint8_t code[kTileRows][kTileCols];
+  __device__ __forceinline__ Cel64 cell(int i, int j) const {
+    return Cel64{f[0][i + 2][j + 2], f[1][i + 2][j + 2], f[2][i + 2][j + 2], f[3][i + 2][j + 2]};
+  }
+  __device__ __forceinline__ uint8_t cd(int i, int j) const { return code[i + 2][j + 2]; }
+  __device__ __forceinline__ bool valid(int i, int j) const {
+    return (code[i + 2][j + 2] >> 4) != HB_NODATA_CLASS;
+  }
+};
+template <int DIR>
+__device__ __forceinline__ Fc64 face_forward(const CellTile &T, const BcVals &bc, int ra, int ca) {
+  constexpr int dr = DIR == 0 ? 0 : -1, dc = DIR == 0 ? 1 : 0;  // from A to B
+  const int rb = ra + dr, cb = ca + dc;
+  const Cel64 A = T.cell(ra, ca), B = T.cell(rb, cb);
+  const Cel64 sA = slope64<2, false>(A, T.cell(ra - dr, ca - dc), T.valid(ra - dr, ca - dc), B,
+                                     true);
+  const Cel64 sB = slope64<2, false>(B, A, true, T.cell(rb + dr, cb + dc),
+                                     T.valid(rb + dr, cb + dc));
+  return face64<DIR, 2, false>(bc.type, bc.v, A, T.cd(ra, ca), B, T.cd(rb, cb), sA, sB);
+}
+
+// Pass 1: a block of 32 x 8 cells and nine warps.  The block's cells are staged
+// in shared memory, each face of theirs is evaluated once into shared memory
+// (warps 0-7: the west and north faces of their row's cells; warp 8: the last
+// row of y-faces and the last column of x-faces), then the cells are updated
+// and reversed.  FP64 issue and latency bind it.  512^2 cells, cold: faces in a
+// pass of their own through global memory, IEEE divisions, pow and boundary
+// tables searched by every block 27 + 41 us; one pass 34 us; the step's face,
+// staged cells and three blocks an SM 28 us.
+__global__ void __launch_bounds__(32 * (kCellRows + 1), 3)
 adj_cell_kernel(hb_adjoint_args a) {
   __shared__ BcVals bc;
   __shared__ double red[HB_MAX_ZONES + 1][kCellRows + 1];
   __shared__ double sx[5][kCellRows][33], sy[5][kCellRows + 1][32];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  CellTile &T = *reinterpret_cast<CellTile *>(smem_raw);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const hb_instance &in = *a.instance;
   Grid G{a.instance, a.rows, a.cols, a.pitch, a.code_pitch, a.h, a.qx, a.qy,
@@ -191,20 +211,34 @@ adj_cell_kernel(hb_adjoint_args a) {
   const int rx = extra ? r0 + lane : r, cx = extra ? c0 + 32 : c;
   const bool hasx = (!extra || lane < kCellRows) && rx < a.rows && cx <= a.cols;
   const bool hasy = r <= a.rows && c < a.cols;
-  const bool ghosts = (hasx && is_ghost_face(G, rx, cx - 1, rx, cx)) ||
-                      (hasy && is_ghost_face(G, r, c, r - 1, c));
+  // stage the cells (the dense arrays hold two cells around the raster)
+  for (int q = tid; q < kTileRows * kTileCols; q += 32 * (kCellRows + 1)) {
+    const int i = q / kTileCols, j = q - i * kTileCols;
+    const int rr = r0 + i - 2, cc = c0 + j - 2;
+    Cz v{0, 0, 0, 0};
+    if (rr < a.rows + 2 && cc < a.cols + 2) v = G.cell(rr, cc);
+    T.f[0][i][j] = v.h;
+    T.f[1][i][j] = v.qx;
+    T.f[2][i][j] = v.qy;
+    T.f[3][i][j] = v.z;
+    T.code[i][j] = G.cd(rr, cc);
+  }
+  __syncthreads();
+  const int lx = cx - c0;  // this thread's x-face in the block
+  const bool ghosts = (hasx && T.valid(rx - r0, lx - 1) != T.valid(rx - r0, lx)) ||
+                      (hasy && T.valid(w, lane) != T.valid(w - 1, lane));
   if (__syncthreads_or(ghosts)) {  // boundary tables: blocks with ghost faces only
     load_bc(in, a.t, bc);
     __syncthreads();
   }
   if (hasx) {
-    const FaceOut5 f = face_at<0>(G, bc, rx, cx - 1, rx, cx, nullptr, nullptr, nullptr, nullptr);
-    const int i = rx - r0, j = cx - c0;
+    const Fc64 f = face_forward<0>(T, bc, rx - r0, lx - 1);
+    const int i = rx - r0, j = lx;
     sx[0][i][j] = f.fh; sx[1][i][j] = f.fx; sx[2][i][j] = f.fy; sx[3][i][j] = f.sa;
     sx[4][i][j] = f.sb;
   }
   if (hasy) {
-    const FaceOut5 f = face_at<1>(G, bc, r, c, r - 1, c, nullptr, nullptr, nullptr, nullptr);
+    const Fc64 f = face_forward<1>(T, bc, w, lane);
     sy[0][w][lane] = f.fh; sy[1][w][lane] = f.fx; sy[2][w][lane] = f.fy; sy[3][w][lane] = f.sa;
     sy[4][w][lane] = f.sb;
   }
@@ -214,19 +248,21 @@ adj_cell_kernel(hb_adjoint_args a) {
   if (!extra && r < a.rows && c < a.cols) {
     const size_t k = G.off(r, c);
     double *mu_h = a.mu, *mu_qx = a.mu + a.mu_stride, *mu_qy = a.mu + 2 * a.mu_stride;
-    if (!G.valid(r, c)) {
+    if (!T.valid(w, lane)) {
       a.out_h[k] = a.out_qx[k] = a.out_qy[k] = 0.0;
       mu_h[k] = mu_qx[k] = mu_qy[k] = 0.0;
     } else {
-      const Cz u = G.cell(r, c);
+      const Cel64 u = T.cell(w, lane);
       const C3 ob{a.lam_h[k], a.lam_qx[k], a.lam_qy[k]};
       const double hs = kHs;
       // fluxMask activity (HC/fluxMaskGenerator_Kernel.cu:19-42, cell 0 ignored)
       bool active = a.first || u.h > hs;
-      const int nr[4] = {r, r - 1, r, r + 1}, nc[4] = {c + 1, c, c - 1, c};
-      for (int d = 0; d < 4 && !active; d++) {
-        const bool bug = (nr[d] == in.bug_y && nc[d] == in.bug_x);
-        if (G.valid(nr[d], nc[d]) && !bug && G.cell(nr[d], nc[d]).h > hs) active = true;
+      if (!active) {
+        auto wet = [&](int dr, int dc) {
+          const bool bug = (r + dr == in.bug_y && c + dc == in.bug_x);
+          return T.valid(w + dr, lane + dc) && !bug && T.cell(w + dr, lane + dc).h > hs;
+        };
+        active = wet(0, 1) || wet(-1, 0) || wet(0, -1) || wet(1, 0);
       }
       const double kk = a.dt / in.dx;
       C3 rr{0, 0, 0};
@@ -239,7 +275,7 @@ adj_cell_kernel(hb_adjoint_args a) {
                  sy[3][w][j] + sy[4][w + 1][j]) * kk;
       }
       rr.h += a.rain_rate * a.dt;
-      zone = G.cd(r, c) & 15;
+      zone = T.cd(w, lane) & 15;
       const double n = in.manning[zone];
       CellTape tp;
       const C3 uu{u.h, u.qx, u.qy};
@@ -288,7 +324,7 @@ adj_cell_kernel(hb_adjoint_args a) {
 // evens out the last wave.  Bound by latency at 16 warps an SM (the decision
 // tape of a face fills 128 registers; 156 without the cap, 3 % slower): 62 us a
 // step of 512^2 cells with both directions in one thread and IEEE divisions,
-// 37 us so (cold).
+// 34 us so (cold).
 template <int DIR>
 __device__ __forceinline__ void face_rev_at(const hb_adjoint_args &a, const Grid &G,
                                             const hb_instance &in, BcVals &bc, int r, int c) {
@@ -314,7 +350,7 @@ __device__ __forceinline__ void face_rev_at(const hb_adjoint_args &a, const Grid
     load_bc(in, a.t, bc);
     __syncthreads();
   }
-  if (work) face_at<DIR>(G, bc, ra, ca, rb, cb, &ob, a.out_h, a.out_qx, a.out_qy, a.h_reg);
+  if (work) face_at<DIR>(G, bc, ra, ca, rb, cb, ob, a.out_h, a.out_qx, a.out_qy, a.h_reg);
 }
 
 __global__ void __launch_bounds__(128, 4)
@@ -362,10 +398,12 @@ extern "C" int hb_adjoint_step(const hb_adjoint_args *a, void *stream) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cfg.blockDim = dim3(32, kCellRows + 1);
+  cfg.dynamicSmemBytes = sizeof(CellTile);
   cfg.gridDim = dim3((a->cols + 31) / 32, (a->rows + kCellRows - 1) / kCellRows);
   cudaError_t e = cudaLaunchKernelEx(&cfg, adj_cell_kernel, *a);
   if (e == cudaSuccess) {
     cfg.blockDim = dim3(32, 4);
+    cfg.dynamicSmemBytes = 0;
     cfg.gridDim = dim3((a->cols + 1 + 31) / 32, (a->rows + 1 + 3) / 4, 2);
     e = cudaLaunchKernelEx(&cfg, adj_face_kernel, *a);
   }
