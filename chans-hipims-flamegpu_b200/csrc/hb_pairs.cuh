@@ -1172,30 +1172,32 @@ pairs_mixed_kernel(const hb_instance *__restrict__ insts, const TileEntry *__res
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  // the list is prepare's, several kernels back: read ahead of the wait (2048^2
+  // 79.9 -> 78.5 us a step)
+  TileEntry en = list[min((int)blockIdx.x, n_list - 1)];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   unsigned phase = 0;
   if constexpr (TY != 32) {
     for (int k = blockIdx.x; k < n_list; k += gridDim.x) {
+      if (k != (int)blockIdx.x) en = list[k];
       const bool ok = k >= n_live && k < n_valid_end
-                          ? pair_tile<TY, SOURCES, 1, ORDER>(s, phase, list[k], insts, partials,
+                          ? pair_tile<TY, SOURCES, 1, ORDER>(s, phase, en, insts, partials,
                                                              gparts, gcount, bct, maps)
-                          : pair_tile_general<TY, SOURCES, ORDER>(s, phase, list[k], insts,
-                                                                  partials, gparts, gcount, bct,
-                                                                  maps);
+                          : pair_tile_general<TY, SOURCES, ORDER>(s, phase, en, insts, partials,
+                                                                  gparts, gcount, bct, maps);
       if (!ok) return;
     }
     return;
   }
   const int k = blockIdx.x;
   if (k < n_live || (k >= n_valid_end && k < n_list)) {
-    pair_tile_general<TY, SOURCES, ORDER>(s, phase, list[k], insts, partials, gparts, gcount,
-                                          bct, maps);
+    pair_tile_general<TY, SOURCES, ORDER>(s, phase, en, insts, partials, gparts, gcount, bct,
+                                          maps);
     return;
   }
   if (k < n_valid_end)
-    pair_tile<TY, SOURCES, 1, ORDER>(s, phase, list[k], insts, partials, gparts, gcount, bct,
-                                     maps);
+    pair_tile<TY, SOURCES, 1, ORDER>(s, phase, en, insts, partials, gparts, gcount, bct, maps);
 }
 
 template <int TY, bool SOURCES>
