@@ -2099,8 +2099,9 @@ SideRes g_side[kMaxSideDevices];
 // counts of general tiles (with or without a valid cell) and of the tiles
 // without a valid cell, per prepared workspace (read back at prepare), so
 // that the step launches one CTA per tile; guarded by g_side_mu
+// (and the block count and height it was prepared for)
 struct TileCounts {
-  int general = 0, empty = 0;
+  int general = 0, empty = 0, blocks = 0, rows = 0;
 };
 std::unordered_map<const void *, TileCounts> g_general_tiles;
 
@@ -2226,6 +2227,8 @@ int list_counts(const hb_fused_batch *b, ListCounts &c) {
   if (it == g_general_tiles.end())
     return set_error(HB_ERR_ARG, "hb_fused_step: run hb_fused_prepare on this workspace first");
   c.n = n_blocks(b);
+  if (it->second.blocks != c.n || it->second.rows != step_rows(b))
+    return set_error(HB_ERR_ARG, "hb_fused_step: the batch's tiles changed since hb_fused_prepare");
   const int n_general = std::min(std::max(it->second.general, 0), c.n);
   const int n_empty = std::min(std::max(it->second.empty, 0), n_general);
   c.n_live = n_general - n_empty;
@@ -2524,7 +2527,7 @@ int prepare_impl(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_map
     if (e != cudaSuccess)
       return set_error(HB_ERR_CUDA, "hb_fused_prepare: tile classes: %s", cudaGetErrorString(e));
     std::lock_guard<std::mutex> lock(g_side_mu);
-    g_general_tiles[b->workspace] = TileCounts{counts[0], counts[2]};
+    g_general_tiles[b->workspace] = TileCounts{counts[0], counts[2], n, step_rows(b)};
   }
   // blocks per instance for the volume sum: about 16 cells per thread of the
   // largest instance (the host copy of the records gives the sizes)
@@ -2746,6 +2749,13 @@ namespace {
 template <int TY, bool SOURCES>
 int launch_persistent(const hb_fused_batch *b, int nsteps, long long budget, cudaStream_t st) {
   using S = PairSmem<TY>;
+  {
+    std::lock_guard<std::mutex> lock(g_side_mu);
+    const auto it = g_general_tiles.find(b->workspace);
+    if (it != g_general_tiles.end() &&
+        (it->second.blocks != n_blocks(b) || it->second.rows != step_rows(b)))
+      return set_error(HB_ERR_ARG, "hb_fused_run: the batch's tiles changed since hb_fused_prepare");
+  }
   auto *kern = pairs_persistent_kernel<TY, SOURCES>;
   int rc = set_smem_attr(reinterpret_cast<const void *>(kern), (int)sizeof(S));
   if (rc) return rc;

@@ -72,3 +72,23 @@ def test_blocks_with_sources_strided_grid_and_persistent(cuda):
     _same(a, b)
     _same(a, c)
     _same(a, p)
+
+
+def test_changed_division_without_prepare_is_refused(cuda):
+    """The block height is prepare's: asking for another one afterwards raises
+    instead of stepping on another list, and the solver steps on after it."""
+    from hipims_b200 import scenarios as S
+    from hipims_b200.fused import FusedSolver
+
+    for dtype in (torch.float32, torch.float64):
+        fs = FusedSolver(S.catchment_from(S.urban_catchment(100, seed=2)), dtype=dtype, device=cuda)
+        fs.step(2)
+        fs.batch.flags |= WHOLE
+        with pytest.raises(RuntimeError, match="prepare"):
+            fs.step(1)
+        if dtype == torch.float32:
+            with pytest.raises(RuntimeError, match="prepare"):
+                fs.run_persistent(1)
+        fs.batch.flags &= ~WHOLE
+        fs.step(1)
+        assert fs.controls()[0].step == 3 and fs.controls()[0].status == 0
