@@ -710,10 +710,18 @@ finish_kernel(const hb_instance *__restrict__ insts, BcTable *__restrict__ bct,
 // own class, list entry and partial sums.  Depends on the batch record alone,
 // so that the workspace size, prepare and every step agree.
 // 64-wide FP32 tiles: a CTA's time is its warps' serial walk (8 rows a warp in
-// a 32-row tile, about 1 us a row when the SM holds one CTA), so below one wave
-// of whole tiles 8-row blocks (2 rows a warp) finish sooner although every
-// band start costs an extra row of y-faces.
-constexpr int kDividePairsTiles = 592;
+// a 32-row tile, 1-2 us a row when the SM holds few CTAs), so up to one wave of
+// whole tiles shorter blocks finish sooner although every band start costs an
+// extra row of y-faces: 8-row blocks (2 rows a warp) up to half a wave, 16-row
+// blocks up to one, and up to one and a half where the per-cell source terms
+// make a tile's walk longer.  One 2nd-order step with whole tiles / 16- / 8-row
+// blocks: 256^2 (54 tiles) 25.7 / 15.9 / 14.0 us, 680^2 (253) - / 24.4 / 23.1,
+// 768^2 (350) 32.8 / 25.2 / 27.1, 1000^2 (528) 37.1 / 32.1 / 36.1, 1100^2 (648)
+// 37.3 / 37.4 / 45, 2048^2 (2210) 78 / 89 / 126; with stations and soils
+// 1000^2 44.6 / 37.3 / 42.7, 1000 x 1413 (759) 49.6 / 46.9 / -, 1500^2 (1152)
+// 67.0 / 66.9 / -.
+constexpr int kDividePairs8 = 296, kDividePairs16 = 592;  // 2 and 4 CTAs on each of 148 SMs
+constexpr int kDivideSources16 = 888;
 // FP64 32 x 32 tiles: 16-row blocks (4 rows a warp) put 4 CTAs on an SM and balance
 // the last wave; 8-row blocks up to one of them per CTA slot.  One 2nd-order
 // step with 8- / 16- / 32-row blocks: 100^2 (16 tiles) 13.9 / 17.6 / 25.8 us,
@@ -727,7 +735,10 @@ inline bool is_rows64(const hb_fused_batch *b) {  // the FP64 step kernel (hb_ro
 inline int step_rows(const hb_fused_batch *b) {
   if (b->flags & (HB_FLAG_TILE_TASKS | HB_FLAG_WHOLE_TILES)) return b->tile_y;
   if (is_rows64(b)) return b->n_tiles <= kDivide64Tiles ? 8 : 16;
-  if (b->tile_x == 64 && b->tile_y == 32 && b->n_tiles <= kDividePairsTiles) return 8;
+  if (b->tile_x == 64 && b->tile_y == 32) {
+    const int most = (b->flags & HB_FLAG_SOURCES) ? kDivideSources16 : kDividePairs16;
+    return b->n_tiles <= kDividePairs8 ? 8 : (b->n_tiles <= most ? 16 : 32);
+  }
   return b->tile_y;
 }
 inline int blocks_per_tile(const hb_fused_batch *b) {
@@ -2272,9 +2283,13 @@ int launch_pairs_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   if (lc) return lc;
   const int n = c.n, n_live = c.n_live, n_valid = c.n_valid_end - c.n_live;
   const int n_general = n - n_valid;
-  // 8-row blocks (a small batch): one launch whatever the register cap asked for
+  // 8- and 16-row blocks (a small batch): one launch whatever the register cap
+  // asked for
   if (step_rows(b) == 8)
     return launch_list(pairs_mixed_kernel<8, SOURCES, ORDER>, sizeof(PairSmem<8>), b, nsteps,
+                       b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : n, c, st);
+  if (step_rows(b) == 16)
+    return launch_list(pairs_mixed_kernel<16, SOURCES, ORDER>, sizeof(PairSmem<16>), b, nsteps,
                        b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : n, c, st);
   if (MINB == 4 && b->grid_blocks <= 0)
     return launch_list(pairs_mixed_kernel<TY, SOURCES, ORDER>, sizeof(S), b, nsteps, n, c, st);
@@ -2495,6 +2510,9 @@ int prepare_impl(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_map
     if (b->tile_x == kPW && per == 4)
       classify_tiles_kernel<8, kPW, 4><<<n, kRowsNT, 0, st>>>(b->instances, b->tile_instance, n,
                                                               flags);
+    else if (b->tile_x == kPW && per == 2)
+      classify_tiles_kernel<16, kPW, 2><<<n, kRowsNT, 0, st>>>(b->instances, b->tile_instance, n,
+                                                               flags);
     else if (b->tile_x == kPW)
       classify_tiles_kernel<32, kPW><<<b->n_tiles, kRowsNT, 0, st>>>(
           b->instances, b->tile_instance, b->n_tiles, flags);
@@ -2810,6 +2828,9 @@ extern "C" int hb_fused_run(const hb_fused_batch *b, int nsteps, long long budge
   if (step_rows(b) == 8)
     return src ? launch_persistent<8, true>(b, nsteps, budget, st)
                : launch_persistent<8, false>(b, nsteps, budget, st);
+  if (step_rows(b) == 16)
+    return src ? launch_persistent<16, true>(b, nsteps, budget, st)
+               : launch_persistent<16, false>(b, nsteps, budget, st);
   return src ? launch_persistent<32, true>(b, nsteps, budget, st)
              : launch_persistent<32, false>(b, nsteps, budget, st);
 }

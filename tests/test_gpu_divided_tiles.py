@@ -92,3 +92,24 @@ def test_changed_division_without_prepare_is_refused(cuda):
         fs.batch.flags &= ~WHOLE
         fs.step(1)
         assert fs.controls()[0].step == 3 and fs.controls()[0].status == 0
+
+
+# 16-row blocks: 297 to 592 tiles, to 888 with source terms
+@pytest.mark.parametrize("rows,cols,tiles,soil", [(860, 700, 297, False), (1180, 1020, 592, False),
+                                                  (1180, 1530, 888, True)])
+def test_sixteen_row_blocks_equal_whole_tiles(cuda, rows, cols, tiles, soil):
+    from hipims_b200 import scenarios as S
+
+    d = S.urban_catchment(cols, n_rows=rows, seed=3, rain_mm_h=150.0)
+    c = S.catchment_from(d, **(SOIL if soil else {}))
+    a, b = (_solver([c], cuda, w, origin=(0, 0)) for w in (False, True))
+    assert a.n_tiles == tiles
+    per = a.workspace.numel() / b.workspace.numel()
+    assert per > 1.4  # divided
+    a.step(12)
+    b.step(12)
+    _same(a, b)
+    if not soil:
+        p = _solver([c], cuda, False, origin=(0, 0))
+        p.run_persistent(12)
+        _same(a, p)
