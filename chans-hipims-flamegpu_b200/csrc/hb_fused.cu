@@ -713,15 +713,14 @@ finish_kernel(const hb_instance *__restrict__ insts, BcTable *__restrict__ bct,
 // a 32-row tile, 1-2 us a row when the SM holds few CTAs), so up to one wave of
 // whole tiles shorter blocks finish sooner although every band start costs an
 // extra row of y-faces: 8-row blocks (2 rows a warp) up to half a wave, 16-row
-// blocks up to one, and up to one and a half where the per-cell source terms
-// make a tile's walk longer.  One 2nd-order step with whole tiles / 16- / 8-row
-// blocks: 256^2 (54 tiles) 25.7 / 15.9 / 14.0 us, 680^2 (253) - / 24.4 / 23.1,
-// 768^2 (350) 32.8 / 25.2 / 27.1, 1000^2 (528) 37.1 / 32.1 / 36.1, 1100^2 (648)
-// 37.3 / 37.4 / 45, 2048^2 (2210) 78 / 89 / 126; with stations and soils
-// 1000^2 44.6 / 37.3 / 42.7, 1000 x 1413 (759) 49.6 / 46.9 / -, 1500^2 (1152)
-// 67.0 / 66.9 / -.
+// blocks up to one.  One 2nd-order step with whole tiles / 16- / 8-row blocks:
+// 256^2 (54 tiles) 25.7 / 15.9 / 14.0 us, 680^2 (253) - / 24.4 / 23.1, 768^2
+// (350) 32.8 / 25.2 / 27.1, 1000^2 (528) 37.1 / 32.1 / 36.1, 1100^2 (648) 37.3 /
+// 37.4 / 45, 1180 x 1300 (798) 40.5 / 42.2 / -, 2048^2 (2210) 78 / 89 / 126; with
+// stations and soils 1000^2 44.6 / 37.3 / 42.7.  With those the line could lie at
+// 888 tiles (759: 49.6 / 46.9), but not by HB_FLAG_SOURCES: a batch may set that
+// flag after its workspace was sized or prepared.
 constexpr int kDividePairs8 = 296, kDividePairs16 = 592;  // 2 and 4 CTAs on each of 148 SMs
-constexpr int kDivideSources16 = 888;
 // FP64 32 x 32 tiles: 16-row blocks (4 rows a warp) put 4 CTAs on an SM and balance
 // the last wave; 8-row blocks up to one of them per CTA slot.  One 2nd-order
 // step with 8- / 16- / 32-row blocks: 100^2 (16 tiles) 13.9 / 17.6 / 25.8 us,
@@ -736,8 +735,7 @@ inline int step_rows(const hb_fused_batch *b) {
   if (b->flags & (HB_FLAG_TILE_TASKS | HB_FLAG_WHOLE_TILES)) return b->tile_y;
   if (is_rows64(b)) return b->n_tiles <= kDivide64Tiles ? 8 : 16;
   if (b->tile_x == 64 && b->tile_y == 32) {
-    const int most = (b->flags & HB_FLAG_SOURCES) ? kDivideSources16 : kDividePairs16;
-    return b->n_tiles <= kDividePairs8 ? 8 : (b->n_tiles <= most ? 16 : 32);
+    return b->n_tiles <= kDividePairs8 ? 8 : (b->n_tiles <= kDividePairs16 ? 16 : 32);
   }
   return b->tile_y;
 }

@@ -1,4 +1,4 @@
-"""Small batches step in 8-row blocks of their 32 x 64 tiles (one CTA each)
+"""Small batches step in 8- or 16-row blocks of their 32 x 64 tiles (one CTA each)
 instead of whole tiles: the same arithmetic on every cell, so fields and
 clocks are equal bit for bit to whole tiles (HB_FLAG_WHOLE_TILES); volumes are
 summed in another order (FP32 per lane, then FP64): to 1e-6."""
@@ -94,9 +94,9 @@ def test_changed_division_without_prepare_is_refused(cuda):
         assert fs.controls()[0].step == 3 and fs.controls()[0].status == 0
 
 
-# 16-row blocks: 297 to 592 tiles, to 888 with source terms
+# 16-row blocks: 297 to 592 tiles
 @pytest.mark.parametrize("rows,cols,tiles,soil", [(860, 700, 297, False), (1180, 1020, 592, False),
-                                                  (1180, 1530, 888, True)])
+                                                  (1180, 1020, 592, True)])
 def test_sixteen_row_blocks_equal_whole_tiles(cuda, rows, cols, tiles, soil):
     from hipims_b200 import scenarios as S
 
