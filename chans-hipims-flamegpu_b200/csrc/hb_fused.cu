@@ -747,23 +747,34 @@ inline int n_blocks(const hb_fused_batch *b) {
   return b->n_tiles * std::max(blocks_per_tile(b), 1);
 }
 
-// Workspace layout (each part 256-byte aligned), n = n_blocks: [n]
-// TilePartial, [n_groups] TilePartial (sums of groups of kGroupTiles blocks),
-// [n_groups] unsigned group counters, [n] int32 block order (rows kernel:
-// general blocks, then all-valid blocks), [3] int32 counts, [n] uint8
-// all-valid flags, 64-wide tiles and FP64: [n] TileEntry in the order's order,
-// then [n_instances] BcTable, then [n_instances][kMapsPerInstance]
-// CUtensorMap.  Instance i's groups start at (its first block) / kGroupTiles
-// + i, which never overlaps instance i + 1's.
+// Workspace layout (each part 256-byte aligned): [n_instances] BcTable,
+// [n_instances][kMapsPerInstance] CUtensorMap, the persistent step's 256 bytes;
+// these lie first so that a step of either kernel finds them whichever flags
+// the batch was prepared with.  Then, n = n_blocks: [n] TilePartial, [n_groups]
+// TilePartial (sums of groups of kGroupTiles blocks), [n_groups] unsigned group
+// counters, [n] int32 block order (rows kernel: general blocks, then all-valid
+// blocks), [3] int32 counts, [n] uint8 all-valid flags, 64-wide tiles and FP64:
+// [n] TileEntry in the order's order.  Instance i's groups start at (its first
+// block) / kGroupTiles + i, which never overlaps instance i + 1's.
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-inline size_t ws_partials_bytes(const hb_fused_batch *b) {
-  return align256((size_t)n_blocks(b) * sizeof(TilePartial));
+constexpr int kMapsPerInstance = 9;  // h0 h1 qx0 qx1 qy0 qy1 z h_max code
+constexpr size_t ws_bct_offset(const hb_fused_batch *) { return 0; }
+inline size_t ws_maps_offset(const hb_fused_batch *b) {
+  return align256((size_t)b->n_instances * sizeof(BcTable));
+}
+// the persistent step's counters (3 x uint64)
+inline size_t ws_sync_offset(const hb_fused_batch *b) {
+  return align256(ws_maps_offset(b) + (size_t)b->n_instances * kMapsPerInstance * sizeof(CUtensorMap));
+}
+inline size_t ws_parts_offset(const hb_fused_batch *b) { return ws_sync_offset(b) + 256; }
+inline size_t ws_gparts_offset(const hb_fused_batch *b) {
+  return ws_parts_offset(b) + align256((size_t)n_blocks(b) * sizeof(TilePartial));
 }
 inline int ws_n_groups(const hb_fused_batch *b) {
   return n_blocks(b) / kGroupTiles + b->n_instances + 1;
 }
 inline size_t ws_gcount_offset(const hb_fused_batch *b) {
-  return ws_partials_bytes(b) + align256((size_t)ws_n_groups(b) * sizeof(TilePartial));
+  return ws_gparts_offset(b) + align256((size_t)ws_n_groups(b) * sizeof(TilePartial));
 }
 inline size_t ws_order_offset(const hb_fused_batch *b) {
   return ws_gcount_offset(b) + align256((size_t)ws_n_groups(b) * sizeof(unsigned));
@@ -791,12 +802,6 @@ inline bool has_entries(const hb_fused_batch *b) {
 }
 inline size_t ws_entries_bytes(const hb_fused_batch *b) {
   return has_entries(b) ? align256((size_t)n_blocks(b) * sizeof(TileEntry)) : 0;
-}
-inline size_t ws_bct_offset(const hb_fused_batch *b) {
-  return ws_entries_offset(b) + ws_entries_bytes(b);
-}
-inline size_t ws_maps_offset(const hb_fused_batch *b) {
-  return align256(ws_bct_offset(b) + (size_t)b->n_instances * sizeof(BcTable));
 }
 
 // ---------------------------------------------------------------------------
@@ -1153,7 +1158,6 @@ constexpr int kRowsNT = 32 * kRowsNW;  // threads per CTA
 constexpr int kTW = 32;                // tile width (one warp)
 constexpr int kSWF = kTW + 8;          // staged field row: cols -4..35
 constexpr int kSWC = kTW + 32;         // staged code row: cols -16..47
-constexpr int kMapsPerInstance = 9;    // h0 h1 qx0 qx1 qy0 qy1 z h_max code
 
 template <typename T, int TY>
 struct RowsSmem {
@@ -1973,7 +1977,7 @@ int launch_steps(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   if (blocks_per_sm < 1) blocks_per_sm = 1;
   int grid = b->grid_blocks > 0 ? b->grid_blocks : blocks_per_sm * num_sms();
   if (grid > b->n_tiles) grid = b->n_tiles;
-  TilePartial *parts = reinterpret_cast<TilePartial *>(b->workspace);
+  TilePartial *parts = reinterpret_cast<TilePartial *>((char *)b->workspace + ws_parts_offset(b));
   BcTable *bct = reinterpret_cast<BcTable *>((char *)b->workspace + ws_bct_offset(b));
   for (int k = 0; k < nsteps; k++) {
     fused_step_kernel<T, TY, TX, FAST><<<grid, kNT, sizeof(S), st>>>(
@@ -2165,8 +2169,8 @@ int launch_rows_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   const int grid_a = b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : n;
   const int grid_g = b->grid_blocks > 0 ? std::min(b->grid_blocks, n) : std::min(n_general, n);
   char *ws = reinterpret_cast<char *>(b->workspace);
-  TilePartial *parts = reinterpret_cast<TilePartial *>(ws);
-  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b));
+  TilePartial *parts = reinterpret_cast<TilePartial *>(ws + ws_parts_offset(b));
+  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_gparts_offset(b));
   unsigned *gcount = reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b));
   const int32_t *order = reinterpret_cast<const int32_t *>(ws + ws_order_offset(b));
   const int32_t *counts = reinterpret_cast<const int32_t *>(ws + ws_counts_offset(b));
@@ -2218,8 +2222,8 @@ int launch_list(K *kernel, size_t smem, const hb_fused_batch *b, int nsteps, int
   for (int k = 0; k < nsteps; k++) {
     const cudaError_t e = cudaLaunchKernelEx(
         &cfg, kernel, b->instances, reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b)),
-        c.n_live, c.n_valid_end, c.n, reinterpret_cast<TilePartial *>(ws),
-        reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b)),
+        c.n_live, c.n_valid_end, c.n, reinterpret_cast<TilePartial *>(ws + ws_parts_offset(b)),
+        reinterpret_cast<TilePartial *>(ws + ws_gparts_offset(b)),
         reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b)),
         reinterpret_cast<BcTable *>(ws + ws_bct_offset(b)),
         reinterpret_cast<const CUtensorMap *>(ws + ws_maps_offset(b)), extra...);
@@ -2292,8 +2296,8 @@ int launch_pairs_impl(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   if (MINB == 4 && b->grid_blocks <= 0)
     return launch_list(pairs_mixed_kernel<TY, SOURCES, ORDER>, sizeof(S), b, nsteps, n, c, st);
   char *ws = reinterpret_cast<char *>(b->workspace);
-  TilePartial *parts = reinterpret_cast<TilePartial *>(ws);
-  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b));
+  TilePartial *parts = reinterpret_cast<TilePartial *>(ws + ws_parts_offset(b));
+  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_gparts_offset(b));
   unsigned *gcount = reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b));
   const TileEntry *entries = reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b));
   BcTable *bct = reinterpret_cast<BcTable *>(ws + ws_bct_offset(b));
@@ -2437,14 +2441,11 @@ int encode_maps(const hb_fused_batch *b, cudaStream_t st, CUtensorMap *host_maps
 
 using namespace hb;
 
-// the persistent step's counters (3 x uint64), after the tensor maps
-inline size_t ws_sync_offset(const hb_fused_batch *b) {
-  return align256(ws_maps_offset(b) + (size_t)b->n_instances * kMapsPerInstance * sizeof(CUtensorMap));
-}
-
 extern "C" size_t hb_fused_workspace_size(const hb_fused_batch *b) {
   if (!b) return 0;
-  return ws_sync_offset(b) + 256;
+  hb_fused_batch rows = *b;  // the tile-task kernel takes no more than the rows kernel
+  rows.flags &= ~HB_FLAG_TILE_TASKS;
+  return ws_entries_offset(&rows) + ws_entries_bytes(&rows);
 }
 
 namespace hb {
@@ -2787,8 +2788,8 @@ int launch_persistent(const hb_fused_batch *b, int nsteps, long long budget, cud
   const TileEntry *entries = reinterpret_cast<const TileEntry *>(ws + ws_entries_offset(b));
   const int32_t *counts = reinterpret_cast<const int32_t *>(ws + ws_counts_offset(b));
   const uint8_t *allvalid = reinterpret_cast<const uint8_t *>(ws + ws_flags_offset(b));
-  TilePartial *parts = reinterpret_cast<TilePartial *>(ws);
-  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_partials_bytes(b));
+  TilePartial *parts = reinterpret_cast<TilePartial *>(ws + ws_parts_offset(b));
+  TilePartial *gparts = reinterpret_cast<TilePartial *>(ws + ws_gparts_offset(b));
   unsigned *gcount = reinterpret_cast<unsigned *>(ws + ws_gcount_offset(b));
   BcTable *bct = reinterpret_cast<BcTable *>(ws + ws_bct_offset(b));
   const CUtensorMap *maps = reinterpret_cast<const CUtensorMap *>(ws + ws_maps_offset(b));

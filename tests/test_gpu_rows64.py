@@ -80,3 +80,20 @@ def test_dry_cells_and_limiter_follow_the_oracle(cuda):
     got = fs.compacted(0)
     for f in ("h", "qx", "qy"):
         np.testing.assert_allclose(got[f], sim.state()[f], rtol=0, atol=1e-10, err_msg=f)
+
+
+def test_tile_tasks_asked_for_after_prepare(cuda):
+    """The other kernel's step on a batch prepared for this one: boundary
+    values, maps and partial sums lie where both look for them."""
+    from hipims_b200 import scenarios as S
+
+    c = S.catchment_from(S.urban_catchment(200, n_rows=150, seed=4, rain_mm_h=150.0))
+    a, b = _solver(c, cuda), _solver(c, cuda, kernel="tasks", tile=(32, 32))
+    assert a.batch.tile_x == 32 and a.batch.tile_y == 32
+    a.batch.flags |= 2  # HB_FLAG_TILE_TASKS
+    for s in (a, b):
+        s.step(10)
+    x, y = a.compacted(0), b.compacted(0)
+    for f in x:
+        np.testing.assert_array_equal(x[f], y[f], err_msg=f)
+    assert (a.controls()[0].t, a.controls()[0].step) == (b.controls()[0].t, 10)

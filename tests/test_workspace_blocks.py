@@ -36,3 +36,8 @@ def test_divided_tiles_take_a_larger_workspace(tile, dtype, tiles):
 
 def test_large_fp32_batches_are_not_divided():
     assert _size(593, 1, (32, 64), _lib.HB_F32) == _size(593, 1, (32, 64), _lib.HB_F32, WHOLE)
+
+
+def test_size_does_not_depend_on_the_kernel_asked_for():
+    tasks = 2  # HB_FLAG_TILE_TASKS: may be set or cleared after the workspace was sized
+    assert _size(500, 3, (32, 32), _lib.HB_F64, tasks) == _size(500, 3, (32, 32), _lib.HB_F64)
