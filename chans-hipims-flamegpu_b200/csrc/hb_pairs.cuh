@@ -103,6 +103,19 @@ __device__ __forceinline__ float ex2a(float x) {
   return r;
 }
 
+// Upwind side of a face: left where the first wave or the contact moves right
+// (0 <= sL or 0 < sM).  Its tangential velocity, and on the right cR clamped at 0 (a
+// predicated maximum; selected, it cost 2048^2 1 % more).
+__device__ __forceinline__ void upwind(float sL, float sM, float vL, float vR, float &cR,
+                                       float &vU) {
+  asm("{.reg .pred p;\n\tsetp.gt.ftz.f32 p, %3, 0f00000000;\n\t"
+      "setp.ge.or.ftz.f32 p, %2, 0f00000000, p;\n\t"
+      "@!p max.ftz.f32 %0, %0, 0f00000000;\n\tselp.f32 %1, %4, %5, p;}"
+      : "+f"(cR), "=f"(vU)
+      : "f"(sL), "f"(sM), "f"(vL), "f"(vR));
+}
+
+constexpr float kMinF = 1.17549435e-38f; // least normal number
 constexpr float kHsF = 1.0e-6f;          // h_small
 constexpr float kGF = 9.81f;             // g
 constexpr float kHalfGF = 0.5f * 9.81f;  // exact: a power-of-two scaling of g
@@ -228,13 +241,18 @@ __device__ __forceinline__ void face_core2(f2 ah, f2 bh, f2 bz, f2 Lh, f2 Lz0, f
   // only the contact speed's sign is used: that of num / den is num * den's
   const f2 sM = mul2(num, den);
   // The star flux with the wave speeds clamped at 0 is the flux of every region:
-  // at sL >= 0 it is FL (sR / sR) and at sR <= 0 FR (sL / sL), equal to the unstarred
-  // fluxes up to the rounding of one reciprocal, and in between it is the star
-  // flux itself.  A face between dry sides has the factor 0.  (Selecting the
-  // region's fluxes took seven more instructions per face: 84.0 us a step on
-  // 2048^2, 79.9 so.)
-  const f2 cL = pk(fminf(sL.x, 0.f), fminf(sL.y, 0.f));
-  const f2 cR = pk(fmaxf(sR.x, 0.f), fmaxf(sR.y, 0.f));
+  // right of the last wave it is FR (sL / sL), equal to the unstarred flux up to
+  // the rounding of one reciprocal, and between the waves the star flux itself;
+  // on the left, with cL one least normal number below 0 (its products with a flux
+  // vanish), it is FL (cR / cR).  A face between dry sides has the factor 0.
+  // Only sides with sM <= 0 clamp sR: beside a thin side the speeds may cross
+  // (sL >= 0 >= sR: FL), or both be negative with sM > 0 (the star flux).
+  // (Selecting the region's fluxes 83.7 us a step on 2048^2; so 80.2; with
+  // sR clamped everywhere 78.0, but 0 / 0 or the wrong flux in those two cases.)
+  const f2 cL = pk(fminf(sL.x, -kMinF), fminf(sL.y, -kMinF));
+  f2 cR = sR, vU;
+  upwind(sL.x, sM.x, vL.x, vR.x, cR.x, vU.x);
+  upwind(sL.y, sM.y, vL.y, vR.y, cR.y, vU.y);
   const f2 dS = sub2(cR, cL);
   const bool dry0 = (hL.x < kHsF && hR.x < kHsF) || dd0;
   const bool dry1 = (hL.y < kHsF && hR.y < kHsF) || dd1;
@@ -245,8 +263,6 @@ __device__ __forceinline__ void face_core2(f2 ah, f2 bh, f2 bz, f2 Lh, f2 Lz0, f
   // the tangential flux is the mass flux times the upwind side's tangential
   // velocity in every region (the reference forms the unstarred ones as
   // u * (v * h); (u * h) * v here: one rounding apart)
-  const f2 vU = pk(0.f <= sL.x || 0.f <= sM.x ? vL.x : vR.x,
-                   0.f <= sL.y || 0.f <= sM.y ? vL.y : vR.y);
   ft = mul2(fh, vU);
 }
 
