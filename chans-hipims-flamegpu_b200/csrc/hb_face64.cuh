@@ -76,16 +76,20 @@ __device__ __forceinline__ void face_core64(double Ah, double Az, double Bh, dou
   const double sR = thinR ? fm(2.0, aL, uL) : max64(ad(uR, aR), ad(us, as));
   const double nL = fm(uL, qL, mu(mu(0.5, gL), hL)), nR = fm(uR, qR, mu(mu(0.5, gR), hR));
   const double pL = mu(hL, sb(uL, sL)), pR = mu(hR, sb(uR, sR));
-  // contact speed sM = num / den: only its sign is needed (den != 0 where a side
-  // is wet)
+  // contact speed sM = num / den: only its sign is needed (0 / 0 counts as
+  // negative, as in the reference; so does 0, where no mass crosses)
   const double num = sb(mu(sL, pR), mu(sR, pL)), den = sb(pR, pL);
-  const bool up = 0.0 <= sL || num == 0.0 ||
-                  (__double2hiint(num) ^ __double2hiint(den)) >= 0;
-  // The star flux with the wave speeds clamped at 0 is the flux of every region
-  // (at sL >= 0 it is FL (sR / sR), at sR <= 0 FR), up to the rounding of one
-  // reciprocal; a face between dry sides has the factor 0
+  const bool left = 0.0 <= sL;
+  const bool up =
+      left || (num != 0.0 && (__double2hiint(num) ^ __double2hiint(den)) >= 0);
+  const bool right = !up && __double2hiint(sR) < 0;
+  // The star flux with the wave speeds 0 and 1 on the left of the waves and -1
+  // and 0 on their right is the flux of every region.  (Each speed clamped at 0
+  // by itself is not: beside a thin side they may cross, sL >= 0 >= sR, which is
+  // 0 / 0, or both be negative with sM > 0.)  A face between dry sides has the
+  // factor 0.
   const bool dd = dryA && dryB;
-  const double cL = __double2hiint(sL) < 0 ? sL : 0.0, cR = pos64(sR);
+  const double cL = left ? 0.0 : (right ? -1.0 : sL), cR = right ? 0.0 : (left ? 1.0 : sR);
   double inv = rcp64(sb(cR, cL));
   if ((hL < hs && hR < hs) || dd) inv = 0.0;
   const double cLR = mu(cL, cR);

@@ -4,6 +4,8 @@ may cross, or lie on one side of zero with the contact on the other.  There the
 reference's two evaluations of a face, one from each cell, differ; the step
 kernels evaluate a face once, from its west or south cell, or from the valid
 cell of a boundary face."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -97,13 +99,17 @@ def _one_step(d):
 # Bounds: dt / dx = 0.05 and four faces a cell.  With depths up to 1e-4 m and
 # speeds up to 4 m/s the terms of a face's flux reach 8e-4 (mass) and 5e-3
 # (momentum), each good to a few 1e-7 in FP32 and a few 1e-16 in FP64.
-@pytest.mark.parametrize("dtype,tol_h,tol_q", [(torch.float32, 5e-10, 3e-9)])
+TOL = {torch.float32: (5e-10, 3e-9), torch.float64: (1e-17, 1e-16)}
+
+
+@pytest.mark.parametrize("dtype,wall", [(torch.float32, 30), (torch.float32, 40),
+                                        (torch.float32, 50), (torch.float64, 50)])
 @pytest.mark.parametrize("order", [1, 2])
-@pytest.mark.parametrize("wall", [30, 40, 50])
-def test_films_at_the_dry_depth(cuda, dtype, tol_h, tol_q, order, wall):
+def test_films_at_the_dry_depth(cuda, dtype, wall, order):
     from hipims_b200 import scenarios as S
     from hipims_b200.fused import FusedSolver
 
+    tol_h, tol_q = TOL[dtype]
     for seed in range(3):
         d = _films(200, 10 * wall + seed, wall)
         h, qx, qy = _one_step(d)
@@ -145,3 +151,28 @@ def test_film_moving_off_a_wall(cuda, dtype):
         for f in ("qx", "qy"):
             assert np.all(np.isfinite(got[f]))
             np.testing.assert_allclose(got[f][sure], ref[f][sure], rtol=0, atol=tol, err_msg=f)
+
+
+def test_gradient_through_films(cuda):
+    """The adjoint's forward faces (the step's) and its reverse tape on the same
+    films, against a central difference in the Manning number."""
+    from hipims_b200 import scenarios as S
+    from hipims_b200.adjoint import GaugeMisfit
+
+    d = _films(64, 3, 40)
+    d["manning"] = [0.02]
+    rr, cc = np.nonzero(d["mask"] > 0)
+    nsteps = 2  # the Manning number acts on the first step's discharges, so on the depths of the second
+    p = GaugeMisfit(S.catchment_from(d), rr, cc, nsteps, np.full(nsteps, 0.1), every=1,
+                    checkpoint=2, obs=np.zeros((nsteps, rr.size)), device=cuda,
+                    h_reg=-math.inf)
+
+    def J(n):
+        return float(p.loss(p.simulate([n], 1.0)))
+
+    J(0.02)
+    g = p.gradient()
+    assert np.all(np.isfinite(np.asarray(g)))
+    eps = 2e-7
+    fd = (J(0.02 + eps) - J(0.02 - eps)) / (2 * eps)
+    assert float(g[0]) == pytest.approx(fd, rel=1e-3)
