@@ -158,7 +158,8 @@ __device__ __forceinline__ Cel64 slope64(const Cel64 &c, const Cel64 &m, bool vm
 
 // Face between A (minus side, code ca) and B (plus side, code cb) along DIR
 // from the cells and their slopes; general tiles: a missing side becomes the
-// other cell's ghost, without reconstruction.
+// other cell's ghost, without reconstruction, and the cell is the minus side, in
+// its outward frame (with crossing wave speeds a face has the minus side's flux).
 template <int DIR, int ORDER, bool ALLV>
 __device__ __forceinline__ Fc64 face64(const int *bctype, const double (*bc)[4], Cel64 A,
                                        uint8_t ca, Cel64 B, uint8_t cb, Cel64 sA, Cel64 sB) {
@@ -170,7 +171,12 @@ __device__ __forceinline__ Fc64 face64(const int *bctype, const double (*bc)[4],
       const int cls = (va ? ca : cb) >> 4;
       Cel64 G;
       rule = ghost64<DIR, ORDER>(bctype[cls], bc[cls], va ? A : B, G);
-      if (va) B = G; else A = G;
+      if (!va) {
+        A = Cel64{B.h, -B.qx, -B.qy, B.z};
+        G.qx = -G.qx;
+        G.qy = -G.qy;
+      }
+      B = G;
       sA = sB = Cel64{0.0, 0.0, 0.0, 0.0};
     }
   }
@@ -203,8 +209,13 @@ __device__ __forceinline__ Fc64 face64(const int *bctype, const double (*bc)[4],
   }
   if constexpr (!ALLV) {
     if (!(va || vb) || !rule) o = Fc64{0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!va) o.sa = 0.0;
-    if (!vb) o.sb = 0.0;
+    if (!va) {
+      o.fh = -o.fh;
+      o.sb = o.sa;
+      o.sa = 0.0;
+    } else if (!vb) {
+      o.sb = 0.0;
+    }
   }
   return o;
 }

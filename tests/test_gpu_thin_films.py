@@ -103,7 +103,8 @@ TOL = {torch.float32: (5e-10, 3e-9), torch.float64: (1e-17, 1e-16)}
 
 
 @pytest.mark.parametrize("dtype,wall", [(torch.float32, 30), (torch.float32, 40),
-                                        (torch.float32, 50), (torch.float64, 50)])
+                                        (torch.float32, 50), (torch.float64, 30),
+                                        (torch.float64, 40), (torch.float64, 50)])
 @pytest.mark.parametrize("order", [1, 2])
 def test_films_at_the_dry_depth(cuda, dtype, wall, order):
     from hipims_b200 import scenarios as S
@@ -126,7 +127,7 @@ def test_films_at_the_dry_depth(cuda, dtype, wall, order):
                                        err_msg=f"{f} {seed}")
 
 
-@pytest.mark.parametrize("dtype", [torch.float32])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 def test_film_moving_off_a_wall(cuda, dtype):
     """A uniform film of exactly h_small that leaves a wall: between the wall's cell
     and its ghost the sides part faster than either can follow."""
