@@ -403,9 +403,9 @@ HB_HD void face_rev(const FaceIn &in, const FaceTape<DIR> &tp, const FaceOut5 &o
     aR_b += 0.5 * base_b;
     uL_b += 0.25 * base_b;
     uR_b -= 0.25 * base_b;
-    // a = sqrt(g h)
-    if (hL > 0.0) Lh_b += aL_b * (0.5 * g) * rcp(tp.aL);
-    if (hR > 0.0) Rh_b += aR_b * (0.5 * g) * rcp(tp.aR);
+    // a = sqrt(g h), 0 on the device for a depth below the normal range
+    if (tp.aL > 0.0) Lh_b += aL_b * (0.5 * g) * rcp(tp.aL);
+    if (tp.aR > 0.0) Rh_b += aR_b * (0.5 * g) * rcp(tp.aR);
     // qxL = uL hL, qyL = vL hL, ...
     uL_b += qxL_b * hL;
     Lh_b += qxL_b * uL + qyL_b * vL;
