@@ -771,6 +771,9 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
     const bool infil = SOURCES && in.cum != nullptr;
     const bool stations = SOURCES && in.rain_station != nullptr;
     const bool few = SOURCES && in.n_stations <= kSmemStations;
+    // a pair's ids and depths are one load each where the arrays are aligned to pairs
+    const bool pairs = SOURCES && ((reinterpret_cast<uintptr_t>(in.rain_station) & 3) |
+                                   (reinterpret_cast<uintptr_t>(in.cum) & 7)) == 0;
     const bool fwd_tile = (y0 < HB_PAD_Y && in.halo_up[0] != nullptr) ||
                           (y0 + TY > in.rows - HB_PAD_Y && in.halo_down[0] != nullptr);
     const f2 r2 = dup(dt / dx);
@@ -787,8 +790,15 @@ __device__ __forceinline__ bool pair_tile(PairSmem<TY> &s, unsigned &phase, cons
       f2 cum2 = dup(0.f);
       if constexpr (SOURCES) {
         const size_t go = (size_t)(y0 + i + HB_PAD_Y) * P + (rx0 + HB_PAD_X);
-        if (stations) ids = __ldg(reinterpret_cast<const unsigned *>(in.rain_station + go));
-        if (infil) cum2 = *reinterpret_cast<const f2 *>((const float *)in.cum + go);
+        const uint16_t *sp = in.rain_station + go;
+        const float *cp = (const float *)in.cum + go;
+        if (pairs) {
+          if (stations) ids = __ldg(reinterpret_cast<const unsigned *>(sp));
+          if (infil) cum2 = *reinterpret_cast<const f2 *>(cp);
+        } else {
+          if (stations) ids = __ldg(sp) | (unsigned)__ldg(sp + 1) << 16;
+          if (infil) cum2 = pk(cp[0], cp[1]);
+        }
       }
       // --- x-direction: neighbours W (col 2j-1) and E (col 2j+2)
       const int kc = V.fi(i, j0);
