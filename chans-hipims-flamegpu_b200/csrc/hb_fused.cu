@@ -1977,7 +1977,10 @@ int launch_steps(const hb_fused_batch *b, int nsteps, cudaStream_t st) {
   if (blocks_per_sm < 1) blocks_per_sm = 1;
   int grid = b->grid_blocks > 0 ? b->grid_blocks : blocks_per_sm * num_sms();
   if (grid > b->n_tiles) grid = b->n_tiles;
-  TilePartial *parts = reinterpret_cast<TilePartial *>((char *)b->workspace + ws_parts_offset(b));
+  // this kernel's workspace may be aligned to 8 bytes only (the rows kernels' tensor
+  // maps need 64): its partials lie at the next 16, the regions behind are not its own
+  const uintptr_t at = reinterpret_cast<uintptr_t>(b->workspace) + ws_parts_offset(b);
+  TilePartial *parts = reinterpret_cast<TilePartial *>((at + 15) & ~(uintptr_t)15);
   BcTable *bct = reinterpret_cast<BcTable *>((char *)b->workspace + ws_bct_offset(b));
   for (int k = 0; k < nsteps; k++) {
     fused_step_kernel<T, TY, TX, FAST><<<grid, kNT, sizeof(S), st>>>(

@@ -51,3 +51,20 @@ def test_stations_and_soils_off_their_pair(cuda, dtype, shape):
     ins.cum.copy_(cum[1:].view_as(ins.cum))  # for compacted()
     _same(a, b)
     assert float(ins.cum.max()) > 0.0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_tile_task_workspace_at_eight_bytes(cuda, dtype):
+    from hipims_b200 import scenarios as S
+    from hipims_b200.fused import FusedSolver
+
+    c = S.catchment_from(S.urban_catchment(150, n_rows=200, seed=5, rain_mm_h=150.0))
+    a, b = (FusedSolver([c], dtype=dtype, device=cuda, kernel="tasks", tile=(32, 32))
+            for _ in range(2))
+    ws = torch.zeros(b.workspace.numel() + 8, dtype=torch.uint8, device=cuda)
+    b.batch.workspace = ws.data_ptr() + 8
+    b.prepare()
+    for s in (a, b):
+        s.step(8)
+    _same(a, b)
+    assert a.controls()[0].volume == b.controls()[0].volume
