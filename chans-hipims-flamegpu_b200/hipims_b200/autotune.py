@@ -3,8 +3,10 @@
 For a batch of catchments it times a few steps of each candidate (cells per
 lane -- 2 with 32 x 64 tiles, 1 with 32 x 32 or 64 x 32 tiles -- tile height and
 resident-CTA count) on scratch copies of the catchments, keeps the fastest,
-and caches the choice in a JSON file keyed by the GPU name, the dtype and the
-batch's shape (number of instances, total cells, largest side).
+and caches the choice in a JSON file keyed by the GPU name, the dtype, the
+batch's shape (number of instances, total cells, largest side) and the version of
+the step kernels (KERNELS), so that a choice made among other kernels is timed
+again.
 
 Each candidate is timed after a spin-up of SPINUP_STEPS untimed steps: the
 first steps from a dry start leave most faces dry, where the one-cell kernel's
@@ -34,6 +36,12 @@ DEFAULT_CANDIDATES = ({"tile": (32, 64), "minb": 4}, {"tile": (32, 64), "minb": 
 SPINUP_STEPS = 16
 
 
+# version of what the candidates launch: raise it when a step kernel or the rule that
+# divides tiles into blocks changes which candidate is the fastest (2: programmatic
+# launches, blocks of 8 and 16 rows)
+KERNELS = 2
+
+
 def cells_per_lane(cfg: dict) -> int:
     return int(cfg["tile"][1]) // 32
 
@@ -49,7 +57,7 @@ def batch_key(catchments: Sequence[Catchment], dtype: torch.dtype, device) -> st
     cells = sum(int(c.mask.size) for c in catchments)
     side = max(max(c.mask.shape) for c in catchments)
     return (f"{name}|{str(dtype).split('.')[-1]}|n={len(catchments)}|cells={cells}|side={side}"
-            f"|spinup={SPINUP_STEPS}")
+            f"|kernels={KERNELS}|spinup={SPINUP_STEPS}")
 
 
 def _load() -> dict:
