@@ -82,19 +82,18 @@ __device__ __forceinline__ void face_core64(double Ah, double Az, double Bh, dou
   const bool left = 0.0 <= sL;
   const bool up =
       left || (num != 0.0 && (__double2hiint(num) ^ __double2hiint(den)) >= 0);
-  const bool right = !up && __double2hiint(sR) < 0;
-  // The star flux with the wave speeds 0 and 1 on the left of the waves and -1
-  // and 0 on their right is the flux of every region.  (Each speed clamped at 0
-  // by itself is not: beside a thin side they may cross, sL >= 0 >= sR, which is
-  // 0 / 0, or both be negative with sM > 0.)  A face between dry sides has the
-  // factor 0.
-  const bool dd = dryA && dryB;
-  const double cL = left ? 0.0 : (right ? -1.0 : sL), cR = right ? 0.0 : (left ? 1.0 : sR);
-  double inv = rcp64(sb(cR, cL));
-  if ((hL < hs && hR < hs) || dd) inv = 0.0;
-  const double cLR = mu(cL, cR);
-  fh = mu(fm(cLR, sb(hR, hL), sb(mu(cR, qL), mu(cL, qR))), inv);
-  fn = mu(fm(cLR, sb(qR, qL), sb(mu(cR, nL), mu(cL, nR))), inv);
+  // the region's flux (wave speeds clamped at 0 in the star flux give it too, but
+  // beside a thin side they may cross, which is 0 / 0, or both be negative with
+  // sM > 0); a face between dry sides has the star flux's factor 0
+  const bool dd = dryA && dryB, dry = (hL < hs && hR < hs) || dd;
+  const bool outL = left && !dry, outR = !up && __double2hiint(sR) < 0 && !dry;
+  double inv = rcp64(sb(sR, sL));
+  if (dry) inv = 0.0;
+  const double sLR = mu(sL, sR);
+  fh = mu(fm(sLR, sb(hR, hL), sb(mu(sR, qL), mu(sL, qR))), inv);
+  fn = mu(fm(sLR, sb(qR, qL), sb(mu(sR, nL), mu(sL, nR))), inv);
+  fh = outL ? qL : (outR ? qR : fh);
+  fn = outL ? nL : (outR ? nR : fn);
   // the tangential flux is the mass flux times the upwind tangential velocity
   ft = mu(fh, up ? vL : vR);
   if (dd) sa = sbt = 0.0;
