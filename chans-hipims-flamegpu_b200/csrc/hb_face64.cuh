@@ -13,7 +13,6 @@ __device__ __forceinline__ double max64(double a, double b) { return a > b ? a :
 __device__ __forceinline__ double min64(double a, double b) { return a < b ? a : b; }
 // max(x, 0) by the sign bit
 __device__ __forceinline__ double pos64(double x) { return __double2hiint(x) < 0 ? 0.0 : x; }
-__device__ __forceinline__ double abs64(double x) { return fabs(x); }
 // minmod(x, y) (HC/flucCal_2ndOrder_jh_improved_Kernel.cu:74-81): the sign test
 // on the sign bits (a zero argument has the smaller magnitude and is selected)
 __device__ __forceinline__ double mm64(double x, double y) {

@@ -714,18 +714,18 @@ finish_kernel(const hb_instance *__restrict__ insts, BcTable *__restrict__ bct,
 // whole tiles shorter blocks finish sooner although every band start costs an
 // extra row of y-faces: 8-row blocks (2 rows a warp) up to half a wave, 16-row
 // blocks up to one.  One 2nd-order step with whole tiles / 16- / 8-row blocks:
-// 256^2 (54 tiles) 25.7 / 15.9 / 14.0 us, 680^2 (253) - / 24.4 / 23.1, 768^2
-// (350) 32.8 / 25.2 / 27.1, 1000^2 (528) 37.1 / 32.1 / 36.1, 1100^2 (648) 37.3 /
-// 37.4 / 45, 1180 x 1300 (798) 40.5 / 42.2 / -, 2048^2 (2210) 78 / 89 / 126; with
-// stations and soils 1000^2 44.6 / 37.3 / 42.7.  With those the line could lie at
-// 888 tiles (759: 49.6 / 46.9), but not by HB_FLAG_SOURCES: a batch may set that
-// flag after its workspace was sized or prepared.
+// 256^2 (54 tiles) 22.1 / 15.7 / 14.2 us, 680^2 (253) 28.8 / 24.6 / 24.6, 768^2
+// (350) 32.8 / 25.2 / 27.9, 1000^2 (528) 37.4 / 31.6 / 36.3, 1100^2 (648) 37.3 /
+// 36.9 / 41.8, 1180 x 1300 (798) 41.3 / 42.3 / 49.9, 2048^2 (2210) 79.5 / 88.4 /
+// 117; with stations and soils 1000 x 1413 (759) 48.7 / 47.2 / 54.9.  With those
+// the line could lie at 888 tiles, but not by HB_FLAG_SOURCES: a batch may set
+// that flag after its workspace was sized or prepared.
 constexpr int kDividePairs8 = 296, kDividePairs16 = 592;  // 2 and 4 CTAs on each of 148 SMs
 // FP64 32 x 32 tiles: 16-row blocks (4 rows a warp) put 4 CTAs on an SM and balance
 // the last wave; 8-row blocks up to one of them per CTA slot.  One 2nd-order
-// step with 8- / 16- / 32-row blocks: 100^2 (16 tiles) 13.9 / 17.6 / 25.8 us,
-// 301 x 517 (170) 24.9 / 25.2 / 32.7, 512^2 (289) 30.6 / 29.7 / 34.8, 1024^2
-// (1089) 82.6 / 68.8 / 70.4, 2048^2 (4225) 279 / 220 / 223.
+// step with 8- / 16- / 32-row blocks: 100^2 (16 tiles) 13.1 / 17.0 / 25.6 us,
+// 301 x 517 (170) 24.6 / 22.2 / 29.7, 512^2 (289) 30.7 / 26.3 / 36.5, 1024^2
+// (1089) 79.9 / 67.2 / 71.4, 2048^2 (4225) 277 / 218 / 226.
 constexpr int kDivide64Tiles = 148;
 inline bool is_rows64(const hb_fused_batch *b) {  // the FP64 step kernel (hb_rows64.cuh)
   return b->dtype == HB_F64 && b->tile_x == 32 && b->tile_y == 32 &&

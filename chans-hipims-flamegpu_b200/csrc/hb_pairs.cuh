@@ -105,7 +105,7 @@ __device__ __forceinline__ float ex2a(float x) {
 
 // Upwind side of a face: left where the first wave or the contact moves right
 // (0 <= sL or 0 < sM).  Its tangential velocity, and on the right cR clamped at 0 (a
-// predicated maximum; selected, it cost 2048^2 1 % more).
+// predicated maximum; as a select it cost 2048^2 2 % more).
 __device__ __forceinline__ void upwind(float sL, float sM, float vL, float vR, float &cR,
                                        float &vU) {
   asm("{.reg .pred p;\n\tsetp.gt.ftz.f32 p, %3, 0f00000000;\n\t"

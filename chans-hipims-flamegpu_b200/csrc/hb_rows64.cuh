@@ -8,10 +8,10 @@
 // HC/timeControl_Kernel.cu:164-198 per cell, HC/fluxMaskGenerator_Kernel.cu:19-42
 // for the activity rule).
 //
-// What bounds it: FP64 issue.  An SM starts 64 FP64 lanes a cycle, and a cell
-// needs about 400 FP64 operations (two faces, eight slopes, one update), so the
-// design spends as few of them as it can and keeps 16 warps an SM to cover
-// their latency:
+// What bounds it: latency and FP64 issue.  An SM starts 64 FP64 lanes a cycle,
+// and a cell needs about 400 FP64 operations (two faces, eight slopes, one
+// update), so the design spends as few of them as it can and keeps 16 warps an
+// SM to cover their latency:
 //  * a CTA of 4 warps owns 32 columns x TY rows staged by TMA, lane = column,
 //    each warp walks TY/4 rows; every face is evaluated once (south faces are
 //    kept for the next row, west faces go to the west lane by shuffle, the
@@ -21,7 +21,9 @@
 //    hardware's approximate seed (hb_fp64.cuh: 3 and 6 FP64 operations
 //    instead of a division of about twelve and a root of about ten), one
 //    reciprocal per edge for both velocities, one for the wave span, dt / dx once
-//    per tile; the contact speed's sign is read off numerator and denominator;
+//    per tile; the contact speed's sign is read off numerator and denominator,
+//    beside the star flux, which the left or right state's flux replaces outside
+//    the waves;
 //  * a missing neighbour is replaced by its ghost state before the face, so
 //    ghost faces go through the same code as interior ones and cost selects
 //    instead of a second, divergent evaluation;
@@ -29,9 +31,9 @@
 //    pipe where that is exact.
 // Measured (B200, 2nd order, steps back to back), against the FP64 build of the
 // one-cell-per-lane kernel it replaced (IEEE divisions, pow, 191-230
-// registers, two launches): 1024^2 282 -> 68 us a step, 2048^2 960 -> 220 us,
-// 301 x 517 in 1st order 77 -> 22 us.  1024^2: 41 M warp instructions (81 M
-// before), 15 M of them FP64; issue active 54 %, FP64 pipe 40 %, 16 warps an SM.
+// registers, two launches): 1024^2 282 -> 67 us a step, 2048^2 960 -> 218 us,
+// 301 x 517 in 1st order 77 -> 20 us.  1024^2: 40 M warp instructions (81 M
+// before), 15 M of them FP64; issue active 52 %, FP64 pipe 39 %, 16 warps an SM.
 // Error against 64-bit references of the same steps: unchanged (1.1e-13 of the
 // discharge's norm after 8 steps, set by the reference's friction form).
 // Every operation is pinned (__dadd_rn, __dmul_rn, __fma_rn), so a face

@@ -162,7 +162,8 @@ typedef struct hb_fused_batch {
   int32_t flags;             /* HB_FLAG_* bits */
   const hb_instance *instances;  /* device [n_instances] */
   const int32_t *tile_instance;  /* device [n_tiles] */
-  void *workspace;               /* device, hb_fused_workspace_size() bytes */
+  void *workspace;               /* device, hb_fused_workspace_size() bytes, aligned to 64
+                                    (tensor maps; tile-task kernel: to 8) */
   const hb_instance *instances_host; /* host copy of instances (hb_fused_prepare) */
 } hb_fused_batch;
 
